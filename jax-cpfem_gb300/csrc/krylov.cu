@@ -19,6 +19,7 @@
 #include <string>
 
 #include "cpfem_common.cuh"
+#include "krylov_point.cuh"
 #include "reduce.cuh"
 
 namespace cpfem {
@@ -42,6 +43,8 @@ static_assert(sizeof(SolveOut) == 72 && offsetof(SolveOut, true_rs) == 56, "solv
 // asynchronously instead of waiting for the solve
 constexpr int kKrylovTrueResidual = 1;
 constexpr int kKrylovDeferred = 2;
+static_assert(kPointCounterBytes + kPointCellBytes <= sizeof(double) * 2 * 4 * kMaxBlocks,
+              "the barrier counters and reduction cells fit in the partials");
 
 static thread_local SolveOut g_last_solve = {0, 0, 0.0, 0.0, 0.0, 0.0, 0.0, 0, 0, -1.0, 0.0};
 
@@ -1063,6 +1066,26 @@ static int sm_count_and_blocks(const void* fn, int* blocks_per_sm, int* sms, siz
   return CPFEM_OK;
 }
 
+// The launch's report: copied to the caller's pinned memory behind the solve (deferred: read
+// after its next synchronisation of the stream), or waited for here.
+static int finish_solve(const SolveOut* dev_out, int32_t* info, int flags, cpfem_solve_report_t* report,
+                        cudaStream_t s) {
+  if (flags & kKrylovDeferred) {
+    CPFEM_CUDA_TRY(cudaMemcpyAsync(report, dev_out, sizeof(SolveOut), cudaMemcpyDeviceToHost, s));
+    return CPFEM_OK;
+  }
+  SolveOut out;
+  CPFEM_CUDA_TRY(cudaMemcpyAsync(&out, dev_out, sizeof(SolveOut), cudaMemcpyDeviceToHost, s));
+  CPFEM_CUDA_TRY(cudaStreamSynchronize(s));
+  info[0] = out.k;
+  info[1] = (out.rs <= out.atol2) ? 1 : 0;
+  g_last_solve = out;
+  if (out.error) {
+    set_error("BiCGSTAB grid barrier timed out");
+    return CPFEM_ERR_SOLVE;
+  }
+  return CPFEM_OK;
+}
 
 template <bool TRANS>
 static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double* b, double* x, int precond,
@@ -1071,6 +1094,29 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
                         int flags = 0, cpfem_solve_report_t* report = nullptr) {
   KWork w;
   carve(workspace, L.num_nodes, &w);
+  PointPlan plan{};
+  if (precond != 3) {
+    const int rc = point_plan(L.num_nodes, precond, TRANS, grid_blocks, &plan);
+    if (rc != CPFEM_OK) return rc;
+  }
+  if (plan.ok) {
+    PointArgs a{};
+    a.L = L; a.vals = vals; a.b = b; a.x = x;
+    a.phat = w.phat; a.shat = w.shat;
+    a.counters = (unsigned int*)w.partials;
+    a.cells = w.partials + kPointCounterBytes / sizeof(double);
+    a.error = &w.sync->error;
+    a.out = w.out;
+    a.precond = precond; a.maxiter = maxiter; a.max_restarts = max_restarts;
+    a.true_res = (flags & kKrylovTrueResidual) ? 1 : 0;
+    a.tol = tol; a.atol = atol;
+    // one memset over the error word, the report and the one team's counter (neighbours in the
+    // workspace)
+    CPFEM_CUDA_TRY(cudaMemsetAsync(w.sync, 0, (size_t)((char*)w.partials - (char*)w.sync) + 128, s));
+    const int rc = point_launch(plan, TRANS, a, s);
+    if (rc != CPFEM_OK) return rc;
+    return finish_solve(w.out, info, flags, report, s);
+  }
   CPFEM_CUDA_TRY(cudaMemsetAsync(w.sync, 0, sizeof(GridSync), s));
   if (precond == 1 || precond == 2) {
     k_precond_setup<TRANS><<<(unsigned)ceil_div(L.num_nodes, 128), 128, 0, s>>>(L, vals, precond, w.minv);
@@ -1117,23 +1163,7 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
     k_sum_partials<<<1, 32, 0, s>>>(w.partials, kVecBlocks, &w.out->true_rs);
     CPFEM_CUDA_TRY(cudaGetLastError());
   }
-  if (flags & kKrylovDeferred) {
-    // queued behind the solve and the true residual: the caller reads it after its next
-    // synchronisation of the stream
-    CPFEM_CUDA_TRY(cudaMemcpyAsync(report, w.out, sizeof(SolveOut), cudaMemcpyDeviceToHost, s));
-    return CPFEM_OK;
-  }
-  SolveOut out;
-  CPFEM_CUDA_TRY(cudaMemcpyAsync(&out, w.out, sizeof(SolveOut), cudaMemcpyDeviceToHost, s));
-  CPFEM_CUDA_TRY(cudaStreamSynchronize(s));
-  info[0] = out.k;
-  info[1] = (out.rs <= out.atol2) ? 1 : 0;
-  g_last_solve = out;
-  if (out.error) {
-    set_error("BiCGSTAB grid barrier timed out");
-    return CPFEM_ERR_SOLVE;
-  }
-  return CPFEM_OK;
+  return finish_solve(w.out, info, flags, report, s);
 }
 
 static bool sell_ok(const cpfem_sell_t* L) {
@@ -1650,6 +1680,61 @@ __global__ void __launch_bounds__(kPThreads, 4) k_bicgstab_ragged(
   }
 }
 
+// Teams of the shared-memory kernel, one per job: every job's share of the blocks by weight
+// (at least one block, at most one per kMinPointNodes nodes).  Not used (plan->ok = false)
+// where that leaves a job's vectors too large for its blocks, or with more than half as many
+// jobs as SMs: then the FP64 pipe is busy anyway and the streaming kernel's four blocks per
+// SM hide more latency.
+constexpr int64_t kMinPointNodes = 16;
+
+static int ragged_point_plan(const std::vector<RJob>& jobs, const std::vector<double>& wts, int precond,
+                             PointPlan* plan, std::vector<PointTeam>* teams, std::vector<int>* team_of_block) {
+  plan->ok = false;
+  int sms = 0;
+  const int rc = point_max_blocks(&sms);
+  if (rc != CPFEM_OK) return rc;
+  const int nj = (int)jobs.size();
+  if (2 * nj > sms) return CPFEM_OK;
+  double wsum = 0.0;
+  for (double v : wts) wsum += v;
+  int next = 0;
+  int64_t share = 0;
+  for (int j = 0; j < nj; ++j) {
+    const int64_t n = jobs[(size_t)j].n1 - jobs[(size_t)j].n0;
+    int64_t k = 1 + (int64_t)std::floor((double)(sms - nj) * wts[(size_t)j] / wsum);
+    k = std::min<int64_t>(k, std::max<int64_t>(1, ceil_div(n, kMinPointNodes)));
+    teams->push_back(PointTeam{next, (int)k, j, 0, jobs[(size_t)j].n0, jobs[(size_t)j].n1});
+    for (int64_t c = 0; c < k; ++c) team_of_block->push_back(j);
+    next += (int)k;
+    share = std::max(share, ceil_div(n, k));
+  }
+  const int prc = point_plan_teams(share, precond, next, plan);
+  if (prc != CPFEM_OK || !plan->ok) {
+    teams->clear();
+    team_of_block->clear();
+  }
+  return prc;
+}
+
+// The jobs' iteration counts and flags, waited for.
+static int ragged_finish(const RWork& w, const std::vector<RJob>& jobs, int32_t* info, cudaStream_t s) {
+  const int nj = (int)jobs.size();
+  std::vector<int32_t> out((size_t)(2 * nj));
+  int err = 0;
+  CPFEM_CUDA_TRY(cudaMemcpyAsync(out.data(), w.info, sizeof(int32_t) * out.size(), cudaMemcpyDeviceToHost, s));
+  CPFEM_CUDA_TRY(cudaMemcpyAsync(&err, w.error, sizeof(int), cudaMemcpyDeviceToHost, s));
+  CPFEM_CUDA_TRY(cudaStreamSynchronize(s));
+  for (int j = 0; j < nj; ++j) {
+    info[2 * jobs[(size_t)j].inst] = out[(size_t)(2 * j)];
+    info[2 * jobs[(size_t)j].inst + 1] = out[(size_t)(2 * j + 1)];
+  }
+  if (err) {
+    set_error("ragged BiCGSTAB team barrier timed out");
+    return CPFEM_ERR_SOLVE;
+  }
+  return CPFEM_OK;
+}
+
 }  // namespace cpfem
 
 extern "C" {
@@ -1716,9 +1801,32 @@ int cpfem_bicgstab_batched(const cpfem_sell_t* sell, const double* values, const
     set_error("ragged BiCGSTAB kernel cannot be resident");
     return CPFEM_ERR_CUDA;
   }
+  PointPlan plan{};
+  std::vector<PointTeam> pteams;
+  std::vector<int> team_of_block;
+  if (const int prc = ragged_point_plan(jobs, wts, precond, &plan, &pteams, &team_of_block); prc != CPFEM_OK) return prc;
+  if (plan.ok) {
+    PointArgs a{};
+    a.L = *sell; a.vals = values; a.b = b; a.x = x;
+    a.phat = w.phat; a.shat = w.shat;
+    a.counters = (unsigned int*)w.partials;
+    a.cells = w.partials + kPointCounterBytes / sizeof(double);
+    a.error = w.error;
+    a.teams = (PointTeam*)w.teams;
+    a.team_of_block = w.team_of_block;
+    a.info = w.info;
+    a.precond = precond; a.maxiter = maxiter;
+    a.tol = tol; a.atol = atol;
+    CPFEM_CUDA_TRY(cudaMemcpyAsync(w.teams, pteams.data(), sizeof(PointTeam) * pteams.size(), cudaMemcpyHostToDevice, s));
+    CPFEM_CUDA_TRY(cudaMemcpyAsync(w.team_of_block, team_of_block.data(), sizeof(int) * team_of_block.size(),
+                                   cudaMemcpyHostToDevice, s));
+    CPFEM_CUDA_TRY(cudaMemsetAsync(w.partials, 0, kPointCounterBytes, s));
+    CPFEM_CUDA_TRY(cudaMemsetAsync(w.error, 0, sizeof(int), s));
+    if (const int lrc = point_launch(plan, false, a, s); lrc != CPFEM_OK) return lrc;
+    return ragged_finish(w, jobs, info, s);
+  }
   const int bmax = (int)std::min<int64_t>((int64_t)per_sm * sms, kMaxBlocks);
   std::vector<RTeam> teams;
-  std::vector<int> team_of_block;
   if (nj <= bmax) {
     // static plan: one team per job, 1 block plus a share of the spare blocks by weight
     double wsum = 0.0;
@@ -1759,20 +1867,7 @@ int cpfem_bicgstab_batched(const cpfem_sell_t* sell, const double* values, const
   void* args[] = {&Lc, &values, &bb, &xx, &w, &pc, &tl, &at, &mi, &njobs};
   CPFEM_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)k_bicgstab_ragged, dim3((unsigned)blocks), dim3(kPThreads),
                                              args, 0, s));
-  std::vector<int32_t> out((size_t)(2 * nj));
-  int err = 0;
-  CPFEM_CUDA_TRY(cudaMemcpyAsync(out.data(), w.info, sizeof(int32_t) * out.size(), cudaMemcpyDeviceToHost, s));
-  CPFEM_CUDA_TRY(cudaMemcpyAsync(&err, w.error, sizeof(int), cudaMemcpyDeviceToHost, s));
-  CPFEM_CUDA_TRY(cudaStreamSynchronize(s));
-  for (int j = 0; j < nj; ++j) {
-    info[2 * jobs[(size_t)j].inst] = out[(size_t)(2 * j)];
-    info[2 * jobs[(size_t)j].inst + 1] = out[(size_t)(2 * j + 1)];
-  }
-  if (err) {
-    set_error("ragged BiCGSTAB team barrier timed out");
-    return CPFEM_ERR_SOLVE;
-  }
-  return CPFEM_OK;
+  return ragged_finish(w, jobs, info, s);
 }
 
 }  // extern "C"

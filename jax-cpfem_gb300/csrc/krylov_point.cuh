@@ -1,0 +1,60 @@
+// BiCGSTAB with the point preconditioners (none, 1/diag, inverted 3x3 diagonal block) for
+// systems whose vectors fit in the SMs' shared memory: host interface of krylov_point.cu.
+#pragma once
+
+#include "cpfem_common.cuh"
+
+namespace cpfem {
+
+// One team of consecutive blocks and the node range it solves.
+struct PointTeam {
+  int first, nb;      // blocks first .. first + nb - 1
+  int job, pad;       // where the team's report goes (info[2 job], info[2 job + 1])
+  int64_t n0, n1;
+};
+
+constexpr int kPointMaxValues = 3;    // sums per reduction
+constexpr int kPointMaxBlocks = 192;  // blocks of a launch, at most (one per SM)
+// Two buffers of a team's partial sums, and a barrier counter (128 bytes apart) per team.
+constexpr size_t kPointCellBytes = sizeof(double) * 2 * kPointMaxValues * kPointMaxBlocks;
+constexpr size_t kPointCounterBytes = sizeof(unsigned int) * 32 * kPointMaxBlocks;
+
+struct PointArgs {
+  cpfem_sell_t L;
+  const double* vals;
+  const double* b;
+  double* x;
+  double *phat, *shat;          // 3 * num_nodes each: what the neighbours gather
+  double* cells;                // kPointCellBytes
+  unsigned int* counters;       // kPointCounterBytes, zeroed before the launch
+  int* error;                   // zeroed before the launch
+  const PointTeam* teams;       // by team_of_block, or null: one team of all blocks
+  const int* team_of_block;
+  cpfem_solve_report_t* out;    // single system: the launch's report
+  int32_t* info;                // teams: iterations and converged flag per job
+  int precond;
+  int maxiter, max_restarts;
+  int true_res;                 // also form ||b - A x||^2 of the returned x
+  double tol, atol;
+  int smem_bytes;               // dynamic shared memory of a block
+};
+
+// How a solve is laid out: blocks, slot lanes per node; ok = false where the vectors do not
+// fit and the streaming kernel has to run.
+struct PointPlan {
+  bool ok;
+  int blocks;
+  int lanes;
+  int threads;
+  int smem_bytes;
+};
+
+// Plan of one system of n nodes (grid_blocks > 0: that many blocks, at most one per SM).
+int point_plan(int64_t n, int precond, bool transpose, int grid_blocks, PointPlan* plan);
+// Plan of teams whose largest share is max_nodes_per_block nodes.
+int point_plan_teams(int64_t max_nodes_per_block, int precond, int blocks, PointPlan* plan);
+// Blocks of a launch that can be resident together (one per SM).
+int point_max_blocks(int* blocks);
+int point_launch(const PointPlan& plan, bool transpose, PointArgs args, cudaStream_t s);
+
+}  // namespace cpfem
