@@ -386,7 +386,10 @@ typedef struct {
   const int8_t* free_dof;                     /* [3*nodes of level 0]: 0 on Dirichlet dofs */
   double* scratch[2];                         /* Galerkin product in three 1-D passes: stencils of
                                                  the x-coarsened and xy-coarsened operators, each
-                                                 [243*scratch_nodes] */
+                                                 [243*scratch_nodes].  scratch[0] then holds the small
+                                                 coarse levels' part of the cycle as a dense operator
+                                                 until the next set-up (a solve that finds another
+                                                 hierarchy's there smooths the levels itself) */
   int64_t scratch_nodes;                      /* >= max over l of dims_c[0]*dims[l][1]*dims[l][2] */
   int32_t precision;       /* 0: the V-cycle in FP64 on the arrays above; 1: in FP32 on the
                               arrays below (set up from the FP64 operators).  The Krylov
@@ -394,8 +397,8 @@ typedef struct {
                               the right, q = A phat and t = A shat are FP64 products of the
                               actual phat / shat, so r stays the residual of the FP64 system
                               and the stop rule is unchanged; only the iterates differ. */
-  int32_t local_nodes;     /* levels >= 2 with at most this many nodes run inside one block
-                              (0: 256) */
+  int32_t local_nodes;     /* coarse levels with at most this many nodes (0: 256, and at most 256)
+                              are applied as one dense operator formed by the set-up */
   float* values32[CPFEM_MG_MAX_LEVELS];       /* precision 1: the operators of levels >= 1 in
                                                  FP32 (setup); level 0 reads the system's FP64
                                                  values, rounded in registers (may be NULL) */

@@ -1,490 +1,19 @@
-// Persistent BiCGSTAB with the point preconditioners for systems whose Krylov vectors fit in
-// shared memory (up to about 43^3 cells on one GB300): every mesh of the drop-in drivers
-// and the RVEs of a batch.
-//
-// What bounds an iteration at these sizes is latency: five dependencies that cross the grid,
-// and FP64 instructions, which GB300 issues at one warp instruction per 64 cycles and
-// sub-partition, with 65 cycles of latency (a division takes 550).  So
-//  * the nodes are spread over all SMs, one block each, in equal contiguous ranges.  A warp
-//    takes one of the three rows of 32 / QL consecutive nodes, and QL lanes share a row's
-//    neighbour slots.  With one thread per node a 10^3 mesh ran on 6 SMs.
-//  * every vector but the two that neighbours gather lives in the block's shared memory, and
-//    so do, where they fit, the block's matrix rows and column indices (up to ~22^3 cells),
-//    copied once per solve.  A transposed solve copies the transposed rows, so its product
-//    reads shared memory in order like any other.
-//  * FP64 instructions are spent where there is data: one lane computes the scalars, one
-//    warp adds a sum, comparisons of non-negative numbers are integer ones.
-// us per Jacobi iteration on one GB300, one thread per node on n / 256 blocks -> this kernel:
-// 1 cell 30 -> 17, 10^3 57 -> 19, 16^3 60 -> 20, 24^3 60 -> 33, 32^3 61 -> 51, 40^3 116 -> 87.
-// Every sum has a fixed order, so a solve is bitwise reproducible, and all blocks of a team
-// hold the same scalars and take the same branch.  Polls are bounded: a block that waits too
-// long sets the error flag, stops, and the solve returns CPFEM_ERR_SOLVE.
+// Persistent BiCGSTAB with the point preconditioners (none, 1/diag, inverted 3x3 diagonal
+// block) for systems whose Krylov vectors fit in shared memory (up to about 53^3 cells on one
+// GB300): every mesh of the drop-in drivers and the RVEs of a batch.  Plans and launches.
 #include <algorithm>
 #include <cmath>
 
-#include "krylov_point.cuh"
-#include "reduce.cuh"
+#include "krylov_team.cuh"
 
 namespace cpfem {
 
-constexpr int kPtMaxThreads = 768;
-constexpr int kPtMaxWidth = 27;                      // slots per row the plan counts on
-constexpr int kPtSmemBytes = 206 * 1024;             // dynamic shared memory of a block, at most
-constexpr int kPtSpinLimit = 1 << 22;                 // polls of ~0.4 us each: a second or two
-
-struct PtTeam {
-  int first, nb, id;
-  unsigned int seq;   // barriers crossed
-  bool ok;
-};
-
-struct PtShared {
-  double part[kPointMaxValues][kPtMaxThreads];     // the threads' partial sums
-  double sum[kPointMaxValues];
-  double alpha, omega, beta;
-  double rho, rho_new, rs, atol2;                  // thread 0's
-  int bad, steps, k, go, early, restart;
-};
-
-// One warp adds v[0 .. n) in a fixed order; the result is valid in lane 0.
-__device__ __forceinline__ double pt_warp_total(const double* v, int n) {
-  const int lane = threadIdx.x & 31;
-  double a0 = 0.0, a1 = 0.0;
-  int i = lane;
-  for (; i + 32 < n; i += 64) {
-    a0 += v[i];
-    a1 += v[i + 32];
-  }
-  if (i < n) a0 += v[i];
-  double acc[1] = {n > 32 ? a0 + a1 : a0};
-  warp_sum<1>(acc);
-  return acc[0];
-}
-
-// Team-wide sums of NV values, left in sh.sum (NV = 0: a barrier); also publishes every global
-// write the block made before.  The threads below `active` hold partial sums.  The block's
-// total of value k is warp k's work, as is the team's, whose partials every block adds in
-// block order, so all hold the same bits.  The FP64 pipe is why: a warp instruction takes it
-// 64 cycles, and a shuffle tree in all 16 warps costs more of it than the vector work it sums.
-// The barrier is a counter that only grows (zeroed before the launch): one arrival per block,
-// one polling warp per value.
-template <int NV>
-__device__ __forceinline__ void pt_reduce(const double* v, int active, PtTeam& tm, const PointArgs& a, PtShared& sh) {
-  constexpr int NC = NV > 0 ? NV : 1;
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if constexpr (NV > 0) {
-    if ((int)threadIdx.x < active)
-#pragma unroll
-      for (int k = 0; k < NC; ++k) sh.part[k][threadIdx.x] = v[k];
-    __syncthreads();
-  }
-  double* const cells = a.cells + (size_t)(tm.seq & 1) * kPointMaxValues * kPointMaxBlocks;
-  tm.seq += 1;
-  if constexpr (NV > 0) {
-    if (wid < NC) {
-      const double tot = pt_warp_total(sh.part[wid], active);
-      if (lane == 0) {
-        if (tm.nb == 1) sh.sum[wid] = tot;
-        else __stcg(cells + wid * kPointMaxBlocks + blockIdx.x, tot);
-      }
-    }
-  }
-  __syncthreads();
-  if (tm.nb == 1) return;
-  if (wid < NC) {
-    unsigned int* const count = a.counters + 32 * tm.id;
-    const unsigned int target = tm.seq * (unsigned)tm.nb;
-    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(count), "r"(1u) : "memory");
-    if (lane == 0) {
-      unsigned int c;
-      int spins = 0;
-      do {
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
-      } while (c < target && ++spins < kPtSpinLimit);
-      if (c < target) {
-        atomicExch(a.error, 1);
-        sh.bad = 1;
-      }
-    }
-    __syncwarp();
-    if constexpr (NV > 0) {
-      const double* p = cells + wid * kPointMaxBlocks + tm.first;
-      constexpr int kPer = (kPointMaxBlocks + 31) / 32;
-      double c[kPer];
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) c[i] = (lane + 32 * i < tm.nb) ? __ldcg(p + lane + 32 * i) : 0.0;
-      double acc[1] = {c[0]};
-#pragma unroll
-      for (int i = 1; i < kPer; ++i)
-        if (32 * i < tm.nb) acc[0] += c[i];
-      warp_sum<1>(acc);
-      if (lane == 0) sh.sum[wid] = acc[0];
-    }
-  }
-  __syncthreads();
-  if (sh.bad) tm.ok = false;
-}
-
-// a > b for a, b that are sums of squares or NaN (then false), and v == 0, without the FP64 pipe.
-__device__ __forceinline__ bool pt_greater(double a, double b) {
-  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  return x > y && x <= 0x7FF0000000000000ll && y <= 0x7FF0000000000000ll;
-}
-__device__ __forceinline__ bool pt_zero(double v) { return (__double_as_longlong(v) << 1) == 0ll; }
-
-// The block's share of the system and where its copies live.
-struct PtLocal {
-  int64_t n0;        // first node
-  int nn;            // nodes
-  int units;         // groups of 32 / QL nodes
-  int steps;         // slots per lane, at most
-  bool staged;
-  double* mat;       // [unit][row][step][3][32]
-  int* cols;         // [unit][step][32], 3 * node
-};
-
-// The 3x3 block of node nd's slot (of A^T when TRANS): row i, column c at [stride_i i + stride_c c].
-template <bool TRANS>
-__device__ __forceinline__ const double* pt_block(const PointArgs& a, int64_t nd, int64_t goff, int slot) {
-  const int l = (int)(nd & 31);
-  if (!TRANS) return a.vals + 9 * goff + l + 288 * (int64_t)slot;
-  const int64_t col = __ldg(&a.L.cols[goff + 32 * slot + l]);
-  return a.vals + 9 * __ldg(&a.L.group_off[col >> 5]) + (col & 31) + 288 * (int64_t)__ldg(&a.L.tpos[goff + 32 * slot + l]);
-}
-
-// One row of 32 / QL nodes of A x (A^T x): this warp's task, x gathered from global memory.
-// Plain loads: what other blocks wrote is ordered by the reduction's acquire, and a node's
-// neighbours share most of each other's values, which L1 then serves.  Two chains: a row's
-// FMAs are latency where few warps are at work.  Returns the sum in every lane of the node.
-template <bool TRANS, int QL>
-__device__ __forceinline__ double pt_row(const PointArgs& a, const PtLocal& B, const double* x, int unit, int row) {
-  constexpr int NPW = 32 / QL;
-  constexpr int RS = TRANS ? 32 : 96, CS = TRANS ? 96 : 32;   // strides of a block's row, column
-  const int lane = threadIdx.x & 31;
-  const int node = lane % NPW, q = lane / NPW;
-  double acc = 0.0, acc2 = 0.0;
-  if (B.staged) {
-    const double* m = B.mat + ((size_t)(3 * unit + row) * B.steps) * 96 + lane;
-    const int* c = B.cols + (size_t)unit * B.steps * 32 + lane;
-    int j = 0;
-#pragma unroll 2
-    for (; j + 1 < B.steps; j += 2) {
-      const double *xb = x + c[32 * j], *xc = x + c[32 * j + 32];
-      const double x0 = xb[0], x1 = xb[1], x2 = xb[2], y0 = xc[0], y1 = xc[1], y2 = xc[2];
-      acc = fma(m[96 * j], x0, fma(m[96 * j + 32], x1, fma(m[96 * j + 64], x2, acc)));
-      acc2 = fma(m[96 * j + 96], y0, fma(m[96 * j + 128], y1, fma(m[96 * j + 160], y2, acc2)));
-    }
-    if (j < B.steps) {
-      const double* xb = x + c[32 * j];
-      acc = fma(m[96 * j], xb[0], fma(m[96 * j + 32], xb[1], fma(m[96 * j + 64], xb[2], acc)));
-    }
-  } else if (unit * NPW + node < B.nn) {
-    const int64_t nd = B.n0 + (int64_t)unit * NPW + node;
-    const int64_t goff = a.L.group_off[nd >> 5];
-    const int32_t* cols = a.L.cols + goff + (nd & 31);
-    const int w = a.L.group_width[nd >> 5];
-    int j = q;
-#pragma unroll 2
-    for (; j + QL < w; j += 2 * QL) {
-      const double *vb = pt_block<TRANS>(a, nd, goff, j) + RS * row, *vc = pt_block<TRANS>(a, nd, goff, j + QL) + RS * row;
-      const double *xb = x + 3 * (int64_t)__ldg(&cols[32 * j]), *xc = x + 3 * (int64_t)__ldg(&cols[32 * (j + QL)]);
-      const double a0 = __ldg(&vb[0]), a1 = __ldg(&vb[CS]), a2 = __ldg(&vb[2 * CS]);
-      const double b0 = __ldg(&vc[0]), b1 = __ldg(&vc[CS]), b2 = __ldg(&vc[2 * CS]);
-      const double x0 = xb[0], x1 = xb[1], x2 = xb[2], y0 = xc[0], y1 = xc[1], y2 = xc[2];
-      acc = fma(a0, x0, fma(a1, x1, fma(a2, x2, acc)));
-      acc2 = fma(b0, y0, fma(b1, y1, fma(b2, y2, acc2)));
-    }
-    if (j < w) {
-      const double* vb = pt_block<TRANS>(a, nd, goff, j) + RS * row;
-      const double* xb = x + 3 * (int64_t)__ldg(&cols[32 * j]);
-      acc = fma(__ldg(&vb[0]), xb[0], fma(__ldg(&vb[CS]), xb[1], fma(__ldg(&vb[2 * CS]), xb[2], acc)));
-    }
-  }
-  __syncwarp();
-  acc += acc2;
-#pragma unroll
-  for (int o = NPW; o < 32; o <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  return acc;
-}
-
-template <bool TRANS, int QL>
-__global__ void __launch_bounds__(kPtMaxThreads, 1) k_bicgstab_point(const PointArgs a) {
-  constexpr int NPW = 32 / QL;
-  constexpr int RS = TRANS ? 32 : 96, CS = TRANS ? 96 : 32;
-  extern __shared__ __align__(16) unsigned char pt_smem[];
-  __shared__ PtShared sh;
-  const int threads = (int)blockDim.x, warps = threads >> 5;
-  PtTeam tm{0, (int)gridDim.x, 0, 0u, true};
-  int64_t t0 = 0, t1 = a.L.num_nodes;
-  int job = 0;
-  if (a.teams != nullptr) {
-    tm.id = a.team_of_block[blockIdx.x];
-    const PointTeam t = a.teams[tm.id];
-    tm.first = t.first; tm.nb = t.nb; t0 = t.n0; t1 = t.n1; job = t.job;
-  }
-  // this block's units of NPW nodes: an equal share of the team's
-  const int64_t tu = (t1 - t0 + NPW - 1) / NPW;
-  const int64_t rank = (int)blockIdx.x - tm.first;
-  const int64_t u0 = tu * rank / tm.nb, u1 = tu * (rank + 1) / tm.nb;
-  PtLocal B;
-  B.n0 = t0 + u0 * NPW;
-  B.units = (int)(u1 - u0);
-  B.nn = (int)(min(t0 + u1 * NPW, t1) - B.n0);
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nn = B.nn, nd = 3 * nn;
-  const int mw = a.precond == 2 ? 9 : (a.precond == 1 ? 3 : 0);
-  double* r = reinterpret_cast<double*>(pt_smem);
-  double *rhat = r + nd, *p = rhat + nd, *q = p + nd, *t = q + nd, *xs = t + nd, *ph = xs + nd, *sh_ = ph + nd;
-  double* minv = sh_ + nd;
-  if (threadIdx.x == 0) { sh.bad = 0; sh.steps = 0; }
-  __syncthreads();
-  // slots per lane, and whether the block's rows fit beside the vectors
-  for (int k = threadIdx.x; k < nn; k += threads)
-    atomicMax(&sh.steps, (a.L.group_width[(B.n0 + k) >> 5] + QL - 1) / QL);
-  __syncthreads();
-  B.steps = sh.steps;
-  const size_t vec_bytes = sizeof(double) * (8 * (size_t)nd + (size_t)mw * nn);
-  const size_t items = (size_t)B.units * B.steps * 32;
-  B.staged = vec_bytes + items * (9 * sizeof(double) + sizeof(int)) <= (size_t)a.smem_bytes;
-  B.mat = minv + (size_t)mw * nn;
-  B.cols = reinterpret_cast<int*>(B.mat + 9 * items);
-  if (B.staged)
-    for (int it = threadIdx.x; it < (int)items; it += threads) {
-      const int ln = it & 31, us = it >> 5, u = us / B.steps, j = us - u * B.steps;
-      const int k = u * NPW + ln % NPW, slot = ln / NPW + QL * j;
-      const int64_t node = B.n0 + min(k, nn - 1);    // a lane past the end repeats the last node, with zeros
-      const int64_t goff = a.L.group_off[node >> 5];
-      int64_t col = node;
-      double v[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      if (k < nn && slot < a.L.group_width[node >> 5]) {
-        col = a.L.cols[goff + 32 * slot + (node & 31)];
-        const double* vb = pt_block<TRANS>(a, node, goff, slot);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) v[3 * i + c] = __ldg(&vb[RS * i + CS * c]);
-      }
-      B.cols[it] = (int)(3 * col);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) B.mat[((size_t)(3 * u + i) * B.steps + j) * 96 + 32 * c + ln] = v[3 * i + c];
-    }
-  // the preconditioner of the block's nodes, and x
-  for (int k = threadIdx.x; k < nn; k += threads) {
-    const int64_t node = B.n0 + k;
-    if (mw) {
-      const double* v0 = a.vals + 9 * a.L.group_off[node >> 5] + (node & 31) + 288 * (int64_t)a.L.diag_slot[node];
-      if (mw == 3) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) minv[3 * k + i] = 1.0 / v0[32 * 4 * i];
-      } else {
-        double blk[9], bi[9];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) blk[TRANS ? 3 * c + i : 3 * i + c] = v0[32 * (3 * i + c)];
-        inv3(blk, bi);
-#pragma unroll
-        for (int c = 0; c < 9; ++c) minv[9 * k + c] = bi[c];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 3; ++i) xs[3 * k + i] = a.x[3 * node + i];
-  }
-  __syncthreads();
-
-  const int active = min(nd, threads);       // threads with a dof in the vector phases
-  // y = A x for the block's rows, x complete in global memory; ends with every y visible to
-  // the block
-  auto product = [&](const double* x, double* y) {
-    for (int task = wid; task < 3 * B.units; task += warps) {
-      const int u = task / 3, row = task - 3 * u;
-      const double acc = pt_row<TRANS, QL>(a, B, x, u, row);
-      const int k = u * NPW + lane;
-      if (lane < NPW && k < nn) y[3 * k + row] = acc;
-    }
-    __syncthreads();
-  };
-  // out = M v at the block's dofs, in global memory (for the neighbours) and in hat
-  auto precond = [&](const double* v, double* hat, double* out) {
-    if (mw == 9) __syncthreads();
-    for (int d = threadIdx.x; d < nd; d += threads) {
-      double o;
-      if (mw == 0) o = v[d];
-      else if (mw == 3) o = v[d] * minv[d];
-      else {
-        const int n = d / 3;
-        o = fma(minv[3 * d], v[3 * n], fma(minv[3 * d + 1], v[3 * n + 1], minv[3 * d + 2] * v[3 * n + 2]));
-      }
-      hat[d] = o;
-      out[3 * B.n0 + d] = o;
-    }
-  };
-  // r = b - A x; rhat = p = q = r
-  auto start = [&]() {
-    product(a.x, t);
-    double v2[2] = {0.0, 0.0};
-    for (int d = threadIdx.x; d < nd; d += threads) {
-      const double bv = a.b[3 * B.n0 + d];
-      const double rv = bv - t[d];
-      r[d] = rhat[d] = p[d] = q[d] = rv;
-      v2[0] = fma(bv, bv, v2[0]);
-      v2[1] = fma(rv, rv, v2[1]);
-    }
-    pt_reduce<2>(v2, active, tm, a, sh);   // b.b, r.r
-  };
-  // The scalars of the recurrence, its tests and its stop decision are thread 0's work, the
-  // others read what they need from shared memory: a division in all 16 warps takes the FP64
-  // pipe 1.1 us, a comparison 0.13 us.
-  start();
-  int restarts = 0;
-  if (threadIdx.x == 0) {
-    sh.atol2 = fmax(a.tol * a.tol * sh.sum[0], a.atol * a.atol);
-    if (a.out != nullptr && (int)blockIdx.x == tm.first) a.out->bb = sh.sum[0];
-    sh.rs = sh.rho_new = sh.beta = sh.sum[1];
-    sh.rho = sh.alpha = sh.omega = 1.0;
-    sh.k = 0;
-    sh.go = pt_greater(sh.rs, sh.atol2) && a.maxiter > 0;
-  }
-  __syncthreads();
-
-  // restart at the x in global memory: rhat = p = q = r = b - A x
-  auto restart = [&]() {
-    ++restarts;
-    start();
-    if (threadIdx.x == 0) {
-      sh.rs = sh.rho_new = sh.beta = sh.sum[1];
-      sh.rho = sh.alpha = sh.omega = 1.0;
-      sh.go = pt_greater(sh.rs, sh.atol2) && sh.k < a.maxiter;
-    }
-    __syncthreads();
-  };
-
-  double true_rs = -1.0;
-  for (;;) {
-    while (tm.ok && sh.go) {
-      {
-        const double beta = sh.beta, omega = sh.omega;
-        for (int d = threadIdx.x; d < nd; d += threads) p[d] = r[d] + beta * (p[d] - omega * q[d]);
-      }
-      precond(p, ph, a.phat);
-      pt_reduce<0>(nullptr, active, tm, a, sh);
-      product(a.phat, q);
-      double v1[1] = {0.0};
-      for (int d = threadIdx.x; d < nd; d += threads) v1[0] = fma(rhat[d], q[d], v1[0]);
-      pt_reduce<1>(v1, active, tm, a, sh);
-      if (threadIdx.x == 0) sh.alpha = sh.rho_new / sh.sum[0];
-      __syncthreads();
-      const double alpha = sh.alpha;
-      // s = r - alpha q, kept in r; s.s joins the next sums
-      double vt[3] = {0.0, 0.0, 0.0};
-      for (int d = threadIdx.x; d < nd; d += threads) {
-        const double sv = r[d] - alpha * q[d];
-        r[d] = sv;
-        vt[2] = fma(sv, sv, vt[2]);
-      }
-      precond(r, sh_, a.shat);
-      pt_reduce<0>(nullptr, active, tm, a, sh);
-      product(a.shat, t);
-      for (int d = threadIdx.x; d < nd; d += threads) {
-        vt[0] = fma(t[d], r[d], vt[0]);
-        vt[1] = fma(t[d], t[d], vt[1]);
-      }
-      pt_reduce<3>(vt, active, tm, a, sh);
-      if (threadIdx.x == 0) {
-        sh.omega = sh.sum[0] / sh.sum[1];
-        sh.early = pt_greater(sh.atol2, sh.sum[2]);
-      }
-      __syncthreads();
-      const bool early = sh.early != 0;
-      const double omega = sh.omega;
-      double vr[2] = {0.0, 0.0};
-      for (int d = threadIdx.x; d < nd; d += threads) {
-        double rv;
-        if (early) {
-          xs[d] = xs[d] + alpha * ph[d];
-          rv = r[d];
-        } else {
-          xs[d] = xs[d] + (alpha * ph[d] + omega * sh_[d]);
-          rv = r[d] - omega * t[d];
-        }
-        r[d] = rv;
-        vr[0] = fma(rv, rv, vr[0]);
-        vr[1] = fma(rhat[d], rv, vr[1]);
-      }
-      pt_reduce<2>(vr, active, tm, a, sh);
-      if (wid == 0) {
-        // beta = rho_new / rho * alpha / omega, both quotients at once
-        const double num = lane == 1 ? alpha : sh.sum[1], den = lane == 1 ? omega : sh.rho_new;
-        const double f = num / den;
-        const double g = __shfl_sync(0xffffffffu, f, 1);
-        if (lane == 0) {
-          int kn = (pt_zero(omega) || pt_zero(alpha)) ? -11 : sh.k + 1;
-          if (pt_zero(sh.rho_new)) kn = -10;
-          sh.rho = sh.rho_new;
-          sh.rs = sh.sum[0];
-          sh.rho_new = sh.sum[1];
-          sh.beta = f * g;
-          const bool left = pt_greater(sh.rs, sh.atol2);
-          sh.restart = kn < 0 && restarts < a.max_restarts && left;
-          sh.k = sh.restart ? sh.k + 1 : kn;
-          sh.go = left && sh.k < a.maxiter && sh.k >= 0;
-        }
-      }
-      __syncthreads();
-      if (sh.restart && tm.ok) {
-        for (int d = threadIdx.x; d < nd; d += threads) a.x[3 * B.n0 + d] = xs[d];
-        pt_reduce<0>(nullptr, active, tm, a, sh);
-        restart();
-      }
-    }
-    for (int d = threadIdx.x; d < nd; d += threads) a.x[3 * B.n0 + d] = xs[d];
-    if (!(a.true_res || a.max_restarts > 0) || !tm.ok) break;
-    double vt[1] = {0.0};
-    pt_reduce<0>(nullptr, active, tm, a, sh);
-    product(a.x, t);
-    for (int d = threadIdx.x; d < nd; d += threads) {
-      const double rv = a.b[3 * B.n0 + d] - t[d];
-      vt[0] = fma(rv, rv, vt[0]);
-    }
-    pt_reduce<1>(vt, active, tm, a, sh);
-    true_rs = sh.sum[0];
-    // Where restarts are allowed, a recursive residual that met the stop rule while the true one
-    // is ten times above it (a near-singular system drives it through values so large that it
-    // drifts from b - A x) is a breakdown too.
-    if (threadIdx.x == 0)
-      sh.restart = restarts < a.max_restarts && sh.k >= 0 && sh.k < a.maxiter && !pt_greater(sh.rs, sh.atol2) &&
-                   pt_greater(true_rs, 100.0 * sh.atol2);
-    __syncthreads();
-    if (!sh.restart || !tm.ok) break;
-    restart();
-  }
-  if ((int)blockIdx.x == tm.first && threadIdx.x == 0) {
-    if (a.out != nullptr) {
-      a.out->true_rs = a.true_res ? true_rs : -1.0;
-      a.out->restarts = restarts;
-      a.out->k = sh.k;
-      a.out->error = tm.ok ? 0 : 1;
-      a.out->rs = sh.rs;
-      a.out->atol2 = sh.atol2;
-      a.out->rho = sh.rho;
-      a.out->alpha = sh.alpha;
-      a.out->omega = sh.omega;
-    }
-    if (a.info != nullptr) {
-      a.info[2 * job] = sh.k;
-      a.info[2 * job + 1] = (sh.rs <= sh.atol2) ? 1 : 0;
-    }
-  }
-}
-
 static const void* point_kernel(bool transpose, int lanes) {
   if (transpose)
-    return lanes == 8 ? (const void*)k_bicgstab_point<true, 8> : lanes == 4 ? (const void*)k_bicgstab_point<true, 4>
-         : lanes == 2 ? (const void*)k_bicgstab_point<true, 2> : (const void*)k_bicgstab_point<true, 1>;
-  return lanes == 8 ? (const void*)k_bicgstab_point<false, 8> : lanes == 4 ? (const void*)k_bicgstab_point<false, 4>
-       : lanes == 2 ? (const void*)k_bicgstab_point<false, 2> : (const void*)k_bicgstab_point<false, 1>;
+    return lanes == 8 ? (const void*)k_bicgstab_team<true, 8, void, NoMg> : lanes == 4 ? (const void*)k_bicgstab_team<true, 4, void, NoMg>
+         : lanes == 2 ? (const void*)k_bicgstab_team<true, 2, void, NoMg> : (const void*)k_bicgstab_team<true, 1, void, NoMg>;
+  return lanes == 8 ? (const void*)k_bicgstab_team<false, 8, void, NoMg> : lanes == 4 ? (const void*)k_bicgstab_team<false, 4, void, NoMg>
+       : lanes == 2 ? (const void*)k_bicgstab_team<false, 2, void, NoMg> : (const void*)k_bicgstab_team<false, 1, void, NoMg>;
 }
 
 int point_max_blocks(int* blocks) {
@@ -517,18 +46,19 @@ static int point_lanes(int64_t nodes, int blocks) {
   return best;
 }
 
-// 24 warps where a block's rows are streamed from L2 (more loads in flight), 16 where they are
-// staged (a cheaper block barrier).
-// A transposed product that streams gathers its blocks from the neighbours' rows; past 512
-// nodes a block the streaming kernel's four blocks per SM hide that better (48^3 cells,
-// 774 nodes a block: 202 us per iteration here, 182 there; 40^3, 453 nodes: 115 and 129;
-// not transposed 149 and 165 at 48^3).
-static void point_fit(int64_t share, int precond, bool transpose, PointPlan* plan) {
-  plan->ok = point_smem(share, precond, plan->lanes, false) <= (size_t)kPtSmemBytes && !(transpose && share > 512);
-  const size_t all = point_smem(share, precond, plan->lanes, true);
-  const bool staged = all <= (size_t)kPtSmemBytes;
-  plan->smem_bytes = (int)std::max<size_t>(16, staged ? all : point_smem(share, precond, plan->lanes, false));
-  plan->threads = staged ? 512 : kPtMaxThreads;
+// The rest of a plan, the lanes given: rows staged in shared memory where they fit (16 warps), else
+// read from L2 (24 warps, more loads in flight; what shared memory is left is L1's).  A transposed product that does so gathers its blocks from the neighbours' rows; past
+// 512 nodes a block the streaming kernel's four blocks per SM hide that better (48^3 cells, 774
+// nodes a block: 202 us per iteration here, 182 there; 40^3, 453 nodes: 115 and 129).
+static void point_fit(int64_t nodes, int blocks, int precond, bool transpose, bool teams, PointPlan* plan) {
+  const int64_t npw = 32 / plan->lanes;
+  const int64_t share = (ceil_div(ceil_div(nodes, npw), blocks) + (teams ? 1 : 0)) * npw;
+  const size_t most = (size_t)kPtSmemBytes, vec = point_smem(share, precond, plan->lanes, false),
+               all = point_smem(share, precond, plan->lanes, true);
+  const bool staged = all <= most;
+  plan->ok = vec <= most && !(precond != 3 && transpose && !staged && share > 512);
+  plan->threads = precond == 3 ? kMgThreads : staged ? 512 : kPtMaxThreads;
+  plan->smem_bytes = (int)std::max<size_t>(16, staged ? all : plan->ok ? vec : 0);
 }
 
 int point_plan(int64_t n, int precond, bool transpose, int grid_blocks, PointPlan* plan) {
@@ -540,16 +70,22 @@ int point_plan(int64_t n, int precond, bool transpose, int grid_blocks, PointPla
   blocks = std::max<int64_t>(1, std::min<int64_t>(blocks, ceil_div(n, 4)));
   plan->blocks = (int)blocks;
   plan->lanes = point_lanes(n, (int)blocks);
-  const int npw = 32 / plan->lanes;
-  point_fit(ceil_div(ceil_div(n, npw), blocks) * npw, precond, transpose, plan);
+  if (precond == 3) plan->lanes = std::min(plan->lanes, 4);   // the V-cycle's kernels
+  point_fit(n, (int)blocks, precond, transpose, false, plan);
+  if (precond == 3 && plan->smem_bytes < (int)point_smem(ceil_div(n, blocks), precond, 1, true)) {
+    // rows that stream: a unit of three rows per warp, as few lanes per node as keep most of
+    // the eight warps at work
+    plan->lanes = 1;
+    while (plan->lanes < 4 && ceil_div(ceil_div(n, 32 / plan->lanes), blocks) < 6) plan->lanes *= 2;
+    point_fit(n, (int)blocks, precond, transpose, false, plan);
+  }
   return CPFEM_OK;
 }
 
 int point_plan_teams(int64_t max_nodes_per_block, int precond, int blocks, PointPlan* plan) {
   plan->blocks = blocks;
   plan->lanes = point_lanes(max_nodes_per_block, 1);
-  const int npw = 32 / plan->lanes;
-  point_fit((ceil_div(max_nodes_per_block, npw) + 1) * npw, precond, false, plan);
+  point_fit(max_nodes_per_block, 1, precond, false, true, plan);
   return CPFEM_OK;
 }
 
@@ -557,7 +93,8 @@ int point_launch(const PointPlan& plan, bool transpose, PointArgs args, cudaStre
   const void* fn = point_kernel(transpose, plan.lanes);
   args.smem_bytes = plan.smem_bytes;
   CPFEM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kPtSmemBytes));
-  void* pargs[] = {&args};
+  NoMg none;
+  void* pargs[] = {&args, &none};
   CPFEM_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3((unsigned)plan.blocks), dim3((unsigned)plan.threads), pargs,
                                              (size_t)plan.smem_bytes, s));
   return CPFEM_OK;

@@ -1,5 +1,6 @@
-// BiCGSTAB with the point preconditioners (none, 1/diag, inverted 3x3 diagonal block) for
-// systems whose vectors fit in the SMs' shared memory: host interface of krylov_point.cu.
+// Host interface of the persistent BiCGSTAB by teams of blocks (krylov_team.cuh): the point
+// preconditioners for systems whose vectors fit in the SMs' shared memory (krylov_point.cu),
+// and the multigrid V-cycle (krylov_mg.cu).
 #pragma once
 
 #include "cpfem_common.cuh"
@@ -37,6 +38,8 @@ struct PointArgs {
   int true_res;                 // also form ||b - A x||^2 of the returned x
   double tol, atol;
   int smem_bytes;               // dynamic shared memory of a block
+  double* vectors[8];           // multigrid: the Krylov vectors (3 * num_nodes each) where they do not
+                                // fit in shared memory, else null
 };
 
 // How a solve is laid out: blocks, slot lanes per node; ok = false where the vectors do not
@@ -56,5 +59,15 @@ int point_plan_teams(int64_t max_nodes_per_block, int precond, int blocks, Point
 // Blocks of a launch that can be resident together (one per SM).
 int point_max_blocks(int* blocks);
 int point_launch(const PointPlan& plan, bool transpose, PointArgs args, cudaStream_t s);
+
+// The V-cycle-preconditioned solve (krylov_mg.cu): a plan that is not ok streams its vectors
+// (args.vectors).
+int mg_launch(const PointPlan& plan, bool transpose, PointArgs args, const cpfem_mg_t& hierarchy, cudaStream_t s);
+int mg_check(const cpfem_mg_t* mg, const cpfem_sell_t* sell);
+
+inline bool sell_ok(const cpfem_sell_t* L) {
+  return L && L->num_nodes >= 0 && L->group_off && L->group_width && L->cols && L->diag_slot &&
+         L->num_groups == (L->num_nodes + 31) / 32;
+}
 
 }  // namespace cpfem

@@ -322,8 +322,8 @@ class CrystalPlasticity:
         precision="fp32" runs the V-cycle in single precision on rounded copies of the
         operators (the Krylov iteration and its stop rule stay FP64): faster, but not for
         near-singular systems, where ``solver.bicgstab`` falls back to FP64 by itself.
-        Levels from the third on with at most ``local_nodes`` nodes are smoothed inside
-        one block."""
+        Coarse levels with at most ``local_nodes`` nodes (256 at most) are applied as one dense
+        operator, formed by ``mg_setup`` with the sweep counts it is given."""
         if precision not in ("fp64", "fp32"):
             raise ValueError("multigrid precision must be 'fp64' or 'fp32'")
         if getattr(self, "_mg", None) is not None and self._mg_key == max_levels:
