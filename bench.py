@@ -303,9 +303,10 @@ def gp_flops_per_eval(num_slip, iters_mean, tangent=True, fp32_direction=True, f
     (FP64, FP32): per local iteration one residual (tau 12N, power/slip 6N, L_p 18N, 3x3
     products and strain 130) in FP64, and one 6x6 Jacobian (per slip M^T d 18,
     sym(. (x) n) 15, kk pv 6, rank-one update 72; the cubic stiffness once on six columns,
-    ~100) + LU/solve (~230), in FP32 when the local Newton takes FP32 directions (counted
-    so for every iteration: a lower bound of the FP64 work); the tangent (FP64) adds a
-    Jacobian + LU, 6 dP/ds directions (20N+220 each) and 9 columns (~220 each)."""
+    ~100) + LU/solve (~230), in FP32 when the local Newton takes FP32 directions.  Then
+    the warm start's own steps are FP32 too, and one FP64 residual after them is counted
+    (a lower bound of the FP64 work); the tangent adds a Jacobian + LU, 6 dP/ds directions
+    (20N+220 each) and 9 columns (~220 each)."""
     N = num_slip
     residual = 36 * N + 130
     jac = 111 * N + 100
@@ -313,8 +314,9 @@ def gp_flops_per_eval(num_slip, iters_mean, tangent=True, fp32_direction=True, f
     setup = 120 + residual
     tan = (jac + lu + 6 * (20 * N + 220) + 9 * 220) if tangent else 0
     direction = iters_mean * (jac + lu)
-    fp64 = setup + iters_mean * residual + (0 if fp32_tangent else tan) + 60 + (0 if fp32_direction else direction)
-    fp32 = (direction if fp32_direction else 0.0) + (tan if fp32_tangent else 0.0)
+    its64 = min(iters_mean, 1.0) if fp32_direction else iters_mean
+    fp64 = setup + its64 * residual + (0 if fp32_tangent else tan) + 60 + (0 if fp32_direction else direction)
+    fp32 = (direction + (iters_mean - its64) * residual if fp32_direction else 0.0) + (tan if fp32_tangent else 0.0)
     return fp64, fp32
 
 
@@ -782,8 +784,8 @@ def main():
                "unit": "TFLOP/s", "frac": (gp_flops / gp_t / 1e12) / fp64 if gp_t else None, "traffic": None,
                "kernel": "k_gp_eval<N,tangent>", "peak_source": "cpfem_probe_dfma (of measured)",
                "local_iters_mean": its_t, "fp64_flops_per_gp": gp64, "fp32_flops_per_gp": gp32,
-               "note": "FP64 flops counted with every local Newton direction (and, with the FP32 tangent, every "
-                       "tangent) in FP32: a lower bound of the FP64 work"}
+               "note": "FP64 flops counted with one FP64 residual after the FP32 steps, every local Newton direction "
+                       "(and, with the FP32 tangent, every tangent) in FP32: a lower bound of the FP64 work"}
     # the coloured scatter: algorithmic bytes of a tangent scatter (per GP the tangent, the
     # shape gradients and P read once; per cell the read-add-write of its 64 3x3 blocks and
     # 24 residual entries) and of a residual-only one, over the scatter region's time

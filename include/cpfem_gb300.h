@@ -95,7 +95,7 @@ typedef struct {
   double* g_new;              /* [num_slip*num_gp] */
   double* slip_new;           /* [num_slip*num_gp] */
   double* s_out;              /* [9*num_gp] converged second Piola-Kirchhoff S (global frame) */
-  int32_t* iters;             /* [num_gp] local Newton iterations */
+  int32_t* iters;             /* [num_gp] local Newton iterations, FP32 ones included */
   int32_t* status;            /* [1] OR of CPFEM_GP_* bits (caller zeroes it) */
   const int32_t* cell_list;   /* [num_listed] or NULL: with nodal u, evaluate only the 8 GPs
                                  of each listed cell; every output of other GPs is left
@@ -106,7 +106,8 @@ typedef struct {
                                    s_warm + ds/dF : (F - s_f) instead of at s_warm;
                                  2: Newton directions from an FP32 Jacobian / LU while the
                                    Jacobian's scale max_a d(dgamma_a)/d(tau_a) C11 <= 1e4
-                                   (else FP64); the residual, its stop test and the tangent
+                                   (else FP64), and, with s_warm, the start itself improved
+                                   by Newton steps in FP32 alone; the residual, its stop test and the tangent
                                    stay FP64, so the converged state is the same root;
                                  4: the consistent tangent (dP/dF, and ds/dF for the
                                    prediction) in FP32 under the same scale test (else

@@ -7,9 +7,10 @@
 namespace cpfem {
 
 constexpr int kVjpK = 4;   // tangent directions per dual sweep
+constexpr int kVjpThreads = 64;
 
 template <int NS>
-__global__ void __launch_bounds__(64) k_gp_vjp(const MatDev m, const cpfem_vjp_args_t a) {
+__global__ void __launch_bounds__(kVjpThreads) k_gp_vjp(const __grid_constant__ MatDev m, const cpfem_vjp_args_t a) {
   const int64_t gp = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t G = a.num_gp;
   if (gp >= G) return;
@@ -39,7 +40,7 @@ __global__ void __launch_bounds__(64) k_gp_vjp(const MatDev m, const cpfem_vjp_a
 #pragma unroll
       for (int J = 0; J < 3; ++J) F[3 * i + J] = fma(a.u[3 * nb + i], sg[3 * b + J], F[3 * i + J]);
   }
-  double Fpi[9], R[9], th[5], g[NS], ig[NS];
+  double Fpi[9], R[9], th[5], g[NS];
 #pragma unroll
   for (int k = 0; k < 9; ++k) Fpi[k] = a.fpi[k * G + gp];
 #pragma unroll
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(64) k_gp_vjp(const MatDev m, const cpfem_vjp_a
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
     g[s] = a.g[s * G + gp];
-    ig[s] = 1.0 / g[s];
+    GpSlab<NS, kVjpThreads>::ig(s) = 1.0 / g[s];
   }
   // recompute the converged local state from the checkpoint (u, Fp^-1, g and, if kept,
   // the converged S as the local Newton's start)
@@ -64,15 +65,12 @@ __global__ void __launch_bounds__(64) k_gp_vjp(const MatDev m, const cpfem_vjp_a
   mm3(A, R, AR);
   mm3_at(AR, AR, Ct);
   const double cdt = m.ao * a.dt;
-  GPSolve<NS> st;
-  if (a.s_start != nullptr) {
-    double s0[6];
+  GPSolve st;
+  double s0[6];
+  if (a.s_start != nullptr)
 #pragma unroll
     for (int k = 0; k < 6; ++k) s0[k] = a.s_start[k * G + gp];
-    cp_local_newton<NS>(m, cc, Ct, ig, cdt, 1.0 / th[3], st, s0);
-  } else {
-    cp_local_newton<NS>(m, cc, Ct, ig, cdt, 1.0 / th[3], st);
-  }
+  cp_local_newton<NS, kVjpThreads>(m, cc, Ct, cdt, 1.0 / th[3], st, a.s_start != nullptr ? s0 : nullptr);
   // output cotangents
   constexpr int NY = YOut<NS>::kN;
   double ybar[NY];
@@ -159,8 +157,7 @@ extern "C" int cpfem_gp_vjp(const cpfem_material_t* mat, const cpfem_vjp_args_t*
                     a.param_table, "input pointer is null");
   CPFEM_REQUIRE(md.qmode == 0 || md.num_slip % 3 == 0, "qmode 1 needs num_slip % 3 == 0");
   CPFEM_REQUIRE(a.num_nodes > 0 && a.num_rot > 0 && a.num_param > 0, "table sizes must be given");
-  const int threads = 64;
-  const unsigned blocks = (unsigned)ceil_div(a.num_gp, threads);
+  const unsigned blocks = (unsigned)ceil_div(a.num_gp, kVjpThreads);
   cudaStream_t s = (cudaStream_t)stream;
   const void* fn = (md.num_slip == 12) ? (const void*)k_gp_vjp<12> : (const void*)k_gp_vjp<24>;
   // the dual-number sweeps need a large per-thread stack: make sure the limit covers it
@@ -170,10 +167,12 @@ extern "C" int cpfem_gp_vjp(const cpfem_material_t* mat, const cpfem_vjp_args_t*
   CPFEM_CUDA_TRY(cudaDeviceGetLimit(&limit, cudaLimitStackSize));
   const size_t need = attr.localSizeBytes + 1024;
   if (limit < need) CPFEM_CUDA_TRY(cudaDeviceSetLimit(cudaLimitStackSize, need));
+  const size_t smem = md.num_slip == 12 ? GpSlab<12, kVjpThreads>::kBytes : GpSlab<24, kVjpThreads>::kBytes;
+  CPFEM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (md.num_slip == 12)
-    k_gp_vjp<12><<<blocks, threads, 0, s>>>(md, a);
+    k_gp_vjp<12><<<blocks, kVjpThreads, smem, s>>>(md, a);
   else
-    k_gp_vjp<24><<<blocks, threads, 0, s>>>(md, a);
+    k_gp_vjp<24><<<blocks, kVjpThreads, smem, s>>>(md, a);
   CPFEM_CUDA_TRY(cudaGetLastError());
   return CPFEM_OK;
 }

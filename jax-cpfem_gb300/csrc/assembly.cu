@@ -62,16 +62,19 @@ struct TanIn {
 
 // The FP64 consistent tangent where the FP32 one's scale test fails: out of line, so the
 // FP32-tangent kernel's hot code stays small.
-template <int NS, class StoreCol>
-__device__ __noinline__ void cp_tangent_f64_cold(const MatDev& m, Cub cc, TanIn in, GPSolve<NS> st, double idet,
+template <int NS, int TH, class StoreCol>
+__device__ __noinline__ void cp_tangent_f64_cold(const MatDev& m, Cub cc, TanIn in, GPSolve st, double idet,
                                                  StoreCol store) {
-  cp_tangent<NS>(m, cc, in.F, in.G, st, in.H, in.W, in.Y, idet, store);
+  cp_tangent<NS, TH, double>(m, cc, in.F, in.G, st, in.H, in.W, in.Y, idet, store);
 }
+
+constexpr int kGpThreads = 128;
 
 // TMODE: 0 no tangent, 1 FP64 tangent, 2 FP32 tangent (FP64 where the scale test fails)
 // stored in FP64, 3 the same stored in FP32 (tangent32)
 template <int NS, int TMODE>
-__global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_args_t a) {
+__global__ void __launch_bounds__(kGpThreads) k_gp_eval(const __grid_constant__ MatDev m, const cpfem_gp_args_t a) {
+  using Slab = GpSlab<NS, kGpThreads>;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t G = a.num_gp;
   int64_t gp = tid;
@@ -133,21 +136,17 @@ __global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_
     cc.C44 = a.elastic_table[3 * pi + 2];
   }
 
-  double g[NS], ig[NS];
-#pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    g[s] = a.g[s * G + gp];
-    ig[s] = 1.0 / g[s];
-  }
+#pragma unroll 1
+  for (int s = 0; s < NS; ++s) Slab::ig(s) = 1.0 / a.g[s * G + gp];
   double A[9], AR[9], Ct[9];
   mm3(F, Fpi, A);
   mm3(A, R, AR);
   mm3_at(AR, AR, Ct);
 
-  GPSolve<NS> st;
+  GPSolve st;
   const bool predict = a.s_warm != nullptr && a.s_dsdf != nullptr && a.s_f != nullptr;
+  double s0[6];
   if (a.s_warm != nullptr) {
-    double s0[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) s0[k] = a.s_warm[k * G + gp];
     if (predict && (a.local_flags & 1)) {
@@ -159,7 +158,10 @@ __global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_
         for (int k = 0; k < 6; ++k) s0[k] = fma(a.s_dsdf[(6 * kl + k) * G + gp], dF, s0[k]);
       }
     }
-    cp_local_newton<NS>(m, cc, Ct, ig, m.ao * a.dt, 1.0 / xm, st, s0, (a.local_flags & 2) != 0);
+  }
+  cp_local_newton<NS, kGpThreads>(m, cc, Ct, m.ao * a.dt, 1.0 / xm, st, a.s_warm != nullptr ? s0 : nullptr,
+                                  (a.local_flags & 2) != 0);
+  if (a.s_warm != nullptr) {
     if (st.rn <= m.local_tol) {
 #pragma unroll
       for (int k = 0; k < 6; ++k) a.s_warm[k * G + gp] = st.s[k];
@@ -167,8 +169,6 @@ __global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_
 #pragma unroll
         for (int kl = 0; kl < 9; ++kl) a.s_f[kl * G + gp] = F[kl];
     }
-  } else {
-    cp_local_newton<NS>(m, cc, Ct, ig, m.ao * a.dt, 1.0 / xm, st, nullptr, (a.local_flags & 2) != 0);
   }
   if (a.status != nullptr) {
     int bits = 0;
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_
 
   double Gm[9], H[9], W[9], Y[9], P[9], idet;
   mm3(Fpi, R, Gm);
-  cp_stress<NS>(F, Gm, st, H, W, Y, idet, P);
+  cp_stress(F, Gm, st, H, W, Y, idet, P);
   const double w = (a.weight_jxw && a.jxw != nullptr) ? a.jxw[gp] : 1.0;
 
   // every output but the tangent first, so that the tangent computation (the register-
@@ -202,14 +202,11 @@ __global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_
     for (int c = 0; c < 9; ++c) a.fpi_new[c * G + gp] = Fn[c];
   }
   if (a.slip_new != nullptr)
-#pragma unroll
-    for (int s = 0; s < NS; ++s) a.slip_new[s * G + gp] = a.slip[s * G + gp] + st.dg[s];
-  if (a.g_new != nullptr) {
-    double gn[NS];
-    cp_hardening<NS>(m, g, st.dg, hh, t_sat, gss_a, rq, gn);
-#pragma unroll
-    for (int s = 0; s < NS; ++s) a.g_new[s * G + gp] = gn[s];
-  }
+#pragma unroll 2
+    for (int s = 0; s < NS; ++s) a.slip_new[s * G + gp] = a.slip[s * G + gp] + Slab::dg(s);
+  if (a.g_new != nullptr)
+    cp_hardening<NS, kGpThreads>(m, hh, t_sat, gss_a, rq, [&](int s) { return a.g[s * G + gp]; },
+                                 [&](int s, double v) { a.g_new[s * G + gp] = v; });
   if (a.s_out != nullptr) {
     double Sl[9], T1[9], Sg[9];
     Sl[0] = st.s[0]; Sl[4] = st.s[1]; Sl[8] = st.s[2];
@@ -244,8 +241,8 @@ __global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_
         for (int k = 0; k < 6; ++k) dsdf_out[(6 * kl + k) * G + gp] = to_f64(dsdf[k]);
     };
     if constexpr (TMODE >= 2) {
-      if (tangent_f32_ok<NS>(st, cc)) {
-        cp_tangent_t<NS, float>(m, cc, F, Gm, st, H, W, Y, idet, store);
+      if (scale_f32_ok<NS, kGpThreads>(cc)) {
+        cp_tangent<NS, kGpThreads, float>(m, cc, F, Gm, st, H, W, Y, idet, store);
       } else {
         // the FP64 tangent is the cold path here: out of line, inputs by value
         TanIn in;
@@ -253,10 +250,10 @@ __global__ void __launch_bounds__(128) k_gp_eval(const MatDev m, const cpfem_gp_
         for (int k = 0; k < 9; ++k) {
           in.F[k] = F[k]; in.G[k] = Gm[k]; in.H[k] = H[k]; in.W[k] = W[k]; in.Y[k] = Y[k];
         }
-        cp_tangent_f64_cold<NS>(m, cc, in, st, idet, store);
+        cp_tangent_f64_cold<NS, kGpThreads>(m, cc, in, st, idet, store);
       }
     } else {
-      cp_tangent<NS>(m, cc, F, Gm, st, H, W, Y, idet, store);
+      cp_tangent<NS, kGpThreads, double>(m, cc, F, Gm, st, H, W, Y, idet, store);
     }
   }
 }
@@ -445,20 +442,20 @@ __global__ void __launch_bounds__(256) k_segmented_dot(int32_t nseg, const int64
 
 template <int NS>
 static int launch_gp(const MatDev& md, const cpfem_gp_args_t& a, cudaStream_t s) {
-  const int threads = 128;
   const int64_t work = a.cell_list != nullptr ? 8 * (int64_t)a.num_listed : a.num_gp;
   if (work == 0) return CPFEM_OK;
-  const unsigned blocks = (unsigned)ceil_div(work, threads);
-  if (a.tangent32 != nullptr)
-    k_gp_eval<NS, 3><<<blocks, threads, 0, s>>>(md, a);
-  else if (a.tangent != nullptr && (a.local_flags & 4))
-    k_gp_eval<NS, 2><<<blocks, threads, 0, s>>>(md, a);
-  else if (a.tangent != nullptr)
-    k_gp_eval<NS, 1><<<blocks, threads, 0, s>>>(md, a);
-  else
-    k_gp_eval<NS, 0><<<blocks, threads, 0, s>>>(md, a);
-  CPFEM_CUDA_TRY(cudaGetLastError());
-  return CPFEM_OK;
+  const unsigned blocks = (unsigned)ceil_div(work, kGpThreads);
+  const size_t smem = GpSlab<NS, kGpThreads>::kBytes;
+  auto run = [&](auto* kernel) {
+    CPFEM_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<blocks, kGpThreads, smem, s>>>(md, a);
+    CPFEM_CUDA_TRY(cudaGetLastError());
+    return CPFEM_OK;
+  };
+  if (a.tangent32 != nullptr) return run(k_gp_eval<NS, 3>);
+  if (a.tangent != nullptr && (a.local_flags & 4)) return run(k_gp_eval<NS, 2>);
+  if (a.tangent != nullptr) return run(k_gp_eval<NS, 1>);
+  return run(k_gp_eval<NS, 0>);
 }
 
 }  // namespace cpfem
