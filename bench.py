@@ -786,23 +786,22 @@ def main():
                "local_iters_mean": its_t, "fp64_flops_per_gp": gp64, "fp32_flops_per_gp": gp32,
                "note": "FP64 flops counted with one FP64 residual after the FP32 steps, every local Newton direction "
                        "(and, with the FP32 tangent, every tangent) in FP32: a lower bound of the FP64 work"}
-    # the coloured scatter: algorithmic bytes of a tangent scatter (per GP the tangent, the
-    # shape gradients and P read once; per cell the read-add-write of its 64 3x3 blocks and
-    # 24 residual entries) and of a residual-only one, over the scatter region's time
+    # the scatter: algorithmic bytes of a tangent scatter (per GP the tangent, the shape
+    # gradients and P read once; the read-add-write of the matrix and the residual) and of a
+    # residual-only one, over the scatter region's time
     asm_n, asm_ms = regions.get("elem_assemble", (0, 0.0))
     n_tan = regions.get("gp_eval_tangent", (0, 0.0))[0]
     n_res = regions.get("gp_eval_residual", (0, 0.0))[0]
-    E = prob.num_cells
     tan_b = 4 if prob.fp32_tangent else 8
-    bytes_tan = G * (81 * tan_b + 24 * 8 + 9 * 8) + E * (64 * 9 * 8 * 2 + 24 * 8 * 2)
-    bytes_res = G * (24 * 8 + 9 * 8) + E * 24 * 8 * 2
+    bytes_tan = G * (81 * tan_b + 24 * 8 + 9 * 8) + 16 * (prob.num_values + 3 * prob.num_nodes)
+    bytes_res = G * (24 * 8 + 9 * 8) + 16 * 3 * prob.num_nodes
     asm_roof = None
     if asm_ms > 0:
         asm_gbs = (n_tan * bytes_tan + n_res * bytes_res) / (asm_ms * 1e-3) / 1e9
         asm_roof = {"bound": "hbm", "achieved": asm_gbs, "peak": hbm, "unit": "GB/s",
                     "frac": asm_gbs / hbm if hbm else None, "traffic": None,
-                    "kernel": "k_elem_assemble (coloured scatter, %s tangent)" % ("FP32" if prob.fp32_tangent else
-                                                                                "FP64"),
+                    "kernel": "k_node_assemble (scatter gathered by node, %s tangent)" % ("FP32" if prob.fp32_tangent
+                                                                                          else "FP64"),
                     "algorithmic_bytes_per_tangent_scatter": bytes_tan,
                     "algorithmic_bytes_per_residual_scatter": bytes_res, "scatters": [n_tan, n_res],
                     "peak_source": "HBM from MEASURED_PEAKS.json (of measured)"}
@@ -879,7 +878,7 @@ class CountingLib:
     level-0 block inverses, three directional Galerkin passes and a block inversion per
     coarse level, and two FP32 copies per level for the FP32 V-cycle; every other listed
     entry point launches one kernel."""
-    LAUNCHES = {"cpfem_gp_eval": 1, "cpfem_elem_assemble": 1, "cpfem_elem_assemble_ex": 1, "cpfem_apply_dirichlet": 1, "cpfem_dot": 1,
+    LAUNCHES = {"cpfem_gp_eval": 1, "cpfem_elem_assemble": 1, "cpfem_elem_assemble_ex": 1, "cpfem_node_assemble": 1, "cpfem_apply_dirichlet": 1, "cpfem_dot": 1,
                 "cpfem_bc_initial_guess": 1, "cpfem_axpy": 1, "cpfem_spmv": 1, "cpfem_bicgstab": 2,
                 "cpfem_bicgstab_ex": 2, "cpfem_cell_average": 1, "cpfem_segmented_dot": 1,
                 "cpfem_bicgstab_batched": 2, "cpfem_gp_vjp": 1}

@@ -284,6 +284,16 @@ int cpfem_elem_assemble_ex(int32_t num_cells, const int32_t* cells, const double
                            const double* pk1_w, const void* tangent_w,
                            double* residual, double* values, int32_t k_precision, void* stream);
 
+/* The assembly of cpfem_elem_assemble_ex over the whole mesh, gathered by node in one launch:
+ * node n's cells are node_cells[node_ptr[n] .. node_ptr[n+1]), entries 8*cell + local node.
+ * Values and residual are accumulated into, each by one thread in the order of the list, so
+ * the result is bitwise reproducible.  Nodes of no cell are left as they are. */
+int cpfem_node_assemble(int32_t num_cells, int32_t num_nodes, const int32_t* node_ptr,
+                        const int32_t* node_cells, const double* shape_grads,
+                        const cpfem_sell_t* sell, const uint8_t* elem_pos,
+                        const double* pk1_w, const void* tangent_w,
+                        double* residual, double* values, int32_t k_precision, void* stream);
+
 /* Greedy cell colouring (host): cells of one colour share no node.  color [num_cells]. */
 int cpfem_color_cells(int32_t num_cells, const int32_t* cells, int32_t num_nodes, int32_t* color,
                       int32_t* num_colors);

@@ -320,7 +320,7 @@ def _gp_vjp_state(p, mode, u, cell_bar=None, lam_fp=None, lam_g=None, mu=None):
 
 
 def _sol_cotangent(p, f_bar):
-    """The assembly backward: u_bar_a = sum_q F_bar_q grad N_a (the coloured scatter)."""
+    """The assembly backward: u_bar_a = sum_q F_bar_q grad N_a (the scatter)."""
     ub = torch.zeros(p.num_total_dofs_all_vars, dtype=torch.float64, device=p.device)
     p.scatter(f_bar, None, ub, None)
     return ub.reshape(p.num_nodes, 3)

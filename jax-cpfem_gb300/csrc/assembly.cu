@@ -362,6 +362,163 @@ __global__ void __launch_bounds__(128, SPLIT == 2 ? (sizeof(KT) == 4 ? 4 : 2) : 
   }
 }
 
+// ------------------------------------------------------------------------------------
+// The same assembly gathered by node: 64 threads own the matrix row and the residual of one
+// node, so every value is written once, in a fixed order, by one launch over the whole mesh.
+// Bound by the FP64 pipe where the stiffness is FP64 (19,000 FMA a node, 64 cycles per warp
+// instruction), otherwise by the tangent's loads (each of a cell's eight nodes reads it: L1
+// at 59 % of its rate, the tangent in flight 81 loads at a time).  Per tangent pass, before
+// (eight colours of cells, one launch each) and after: FP64 stiffness 430 -> 47 us at 10^3
+// cells, 1.83 -> 1.17 ms at 32^3; FP32 0.43 -> 0.33 ms at 32^3.  A block holds two nodes,
+// next to one another in the layout: one node reads and writes half sectors (FP32, 32^3, all
+// passes of five load steps: 6.7 ms; two 5.2, four 5.4, eight 6.0).
+//
+// The node's cells are taken eight at a time (a structured mesh has no more).  Thread
+// (cell c, GP q) contracts the tangent with its gradient at the node once for all of the
+// cell's eight neighbours (G_ikL = dN_a/dX_J D_iJkL, to shared memory); thread (c, neighbour
+// b) then sums G . dN_b over the eight GPs; the blocks meet in shared memory, where the
+// threads of a row slot add those that elem_pos sends to it, in cell order.
+// ------------------------------------------------------------------------------------
+constexpr int kNodeThreads = 64, kNodeCells = 8, kBlockNodes = 2;
+// a cell's 8 x 27 contractions, padded by one against bank conflicts between cells
+constexpr int kCellG = 8 * 27 + 1;
+
+template <typename KT>
+struct NodeShared {
+  KT G[kNodeCells * kCellG];
+  KT K[64 * 9];
+  unsigned long long mask[256];
+};
+static_assert(32 % kBlockNodes == 0, "a block's nodes lie in one group of the layout");
+
+template <bool WITH_K, typename KT = double, typename TT = double>
+__global__ void __launch_bounds__(kNodeThreads * kBlockNodes, 8 / kBlockNodes)
+k_node_assemble(int32_t num_nodes, const int32_t* __restrict__ node_ptr, const int32_t* __restrict__ node_cells, int64_t G,
+                const double* __restrict__ sg, const int64_t* __restrict__ goff, const int32_t* __restrict__ gwidth,
+                const uint8_t* __restrict__ epos, const double* __restrict__ Pw, const TT* __restrict__ Dw,
+                double* __restrict__ res, double* __restrict__ vals) {
+  __shared__ double sR_[kBlockNodes][3 * kNodeThreads];
+  __shared__ unsigned spos_[kBlockNodes][16];
+  const int node = threadIdx.x / kNodeThreads, t = threadIdx.x % kNodeThreads, c = t >> 3, q = t & 7;
+  double* const sR = sR_[node];
+  unsigned* const spos = spos_[node];
+  NodeShared<KT>* const sh = reinterpret_cast<NodeShared<KT>*>(gp_slab) + (WITH_K ? node : 0);
+  KT* const sG = sh->G;
+  KT* const sK = sh->K;
+  unsigned long long* const smask = sh->mask;
+  const int64_t na0 = (int64_t)blockIdx.x * kBlockNodes, na = na0 + node;
+  int n0 = 0, n1 = 0, most = 0;     // the node's cells; the most of the block's nodes
+#pragma unroll
+  for (int n = 0; n < kBlockNodes; ++n) {
+    if (na0 + n >= num_nodes) break;
+    const int p0 = node_ptr[na0 + n], p1 = node_ptr[na0 + n + 1];
+    most = max(most, p1 - p0);
+    if (n == node) { n0 = p0; n1 = p1; }
+  }
+  int width = 0;
+  int64_t base = 0;
+  if (WITH_K) {     // the block's nodes are neighbours in one 32-node group of the layout
+    width = gwidth[na0 >> 5];
+    base = 9 * goff[na0 >> 5] + (na0 & 31);
+  }
+  double Rr[3] = {0.0, 0.0, 0.0};
+  for (int s0 = 0; s0 < most; s0 += kNodeCells) {
+    const bool on = n0 + s0 + c < n1;
+    const int64_t entry = on ? node_cells[n0 + s0 + c] : 0;     // 8 cell + local node
+    const int64_t e = entry >> 3;
+    const int a = (int)(entry & 7);
+    if (on) {
+      const int64_t gp = e * 8 + q;
+      const double g0 = sg[gp * 24 + 3 * a], g1 = sg[gp * 24 + 3 * a + 1], g2 = sg[gp * 24 + 3 * a + 2];
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+        Rr[i] = fma(Pw[(3 * i) * G + gp], g0, fma(Pw[(3 * i + 1) * G + gp], g1, fma(Pw[(3 * i + 2) * G + gp], g2, Rr[i])));
+      if constexpr (WITH_K) {
+        const KT a0 = to_prec<KT>(g0), a1 = to_prec<KT>(g1), a2 = to_prec<KT>(g2);
+        KT* out = sG + c * kCellG + q * 27;
+        // kRows rows of nine tangent components in flight together
+        constexpr int kRows = sizeof(TT) == 4 ? 9 : 3;
+#pragma unroll
+        for (int r = 0; r < 9; r += kRows) {
+          TT d[9 * kRows];
+#pragma unroll
+          for (int k = 0; k < 9 * kRows; ++k) d[k] = __ldg(Dw + (int64_t)(9 * r + k) * G + gp);
+#pragma unroll
+          for (int i = 0; i < kRows / 3; ++i)
+#pragma unroll
+            for (int kL = 0; kL < 9; ++kL)
+              out[3 * r + 9 * i + kL] = cp_fma(a0, as_kt<KT>(d[27 * i + kL]),
+                                        cp_fma(a1, as_kt<KT>(d[27 * i + 9 + kL]), a2 * as_kt<KT>(d[27 * i + 18 + kL])));
+        }
+      }
+    }
+    if constexpr (WITH_K) {
+      // row slots of (cell, neighbour), four to a word; 255 marks an absent cell (no row slot
+      // has that number: a row holds at most 255)
+      reinterpret_cast<uint8_t*>(spos)[t] = on ? epos[e * 64 + 8 * a + q] : (uint8_t)255;
+      __syncthreads();
+      // which of the 64 blocks belong to slot p
+      for (int p = t; p < width; p += kNodeThreads) {
+        unsigned long long mask = 0;
+#pragma unroll
+        for (int w = 0; w < 16; ++w) {
+          const unsigned eq = __vcmpeq4(spos[w], (unsigned)p * 0x01010101u) & 0x08040201u;
+          mask |= (unsigned long long)((eq | (eq >> 8) | (eq >> 16) | (eq >> 24)) & 15u) << (4 * w);
+        }
+        smask[p] = mask;
+      }
+      if (on) {
+        const int b = q;
+        KT K[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) K[k] = KT(0);
+#pragma unroll 2
+        for (int r = 0; r < 8; ++r) {
+          const double* gb = sg + (e * 8 + r) * 24 + 3 * b;
+          const KT b0 = to_prec<KT>(gb[0]), b1 = to_prec<KT>(gb[1]), b2 = to_prec<KT>(gb[2]);
+          const KT* gm = sG + c * kCellG + r * 27;
+#pragma unroll
+          for (int k = 0; k < 9; ++k)
+            K[k] = cp_fma(gm[3 * k], b0, cp_fma(gm[3 * k + 1], b1, cp_fma(gm[3 * k + 2], b2, K[k])));
+        }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) sK[9 * t + k] = K[k];
+      }
+      __syncthreads();
+      // slot values 9 p + (3 i + k), summed over the slot's blocks
+      for (int w = threadIdx.x; w < 9 * kBlockNodes * width; w += kNodeThreads * kBlockNodes) {
+        const int o = w / kBlockNodes, p = o / 9, comp = o - 9 * p;
+        const NodeShared<KT>& from = reinterpret_cast<const NodeShared<KT>*>(gp_slab)[w % kBlockNodes];
+        unsigned long long mask = from.mask[p];
+        if (mask != 0) {
+          double* v = &vals[base + 32 * (int64_t)o + w % kBlockNodes];
+          double acc = *v;
+          do {
+            acc += to_f64(from.K[9 * (__ffsll((long long)mask) - 1) + comp]);
+            mask &= mask - 1;
+          } while (mask != 0);
+          *v = acc;
+        }
+      }
+      if (s0 + kNodeCells < most) __syncthreads();     // the next cells reuse the shared arrays
+    }
+  }
+  if (res != nullptr) {
+    // 64 partial sums per component: eight threads add eight each, then in a fixed tree
+#pragma unroll
+    for (int i = 0; i < 3; ++i) sR[i * kNodeThreads + t] = Rr[i];
+    __syncthreads();
+    if (t < 24 && na < num_nodes) {
+      double acc = sR[8 * t];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) acc += sR[8 * t + k];
+#pragma unroll
+      for (int d = 4; d > 0; d >>= 1) acc += __shfl_xor_sync(0x00FFFFFFu, acc, d);
+      if ((t & 7) == 0) res[3 * na + (t >> 3)] += acc;
+    }
+  }
+}
+
 // Row elimination for a list of unique Dirichlet dofs.
 __global__ void k_dirichlet(int32_t nbc, const int32_t* __restrict__ dofs, const double* __restrict__ bvals,
                             const double* __restrict__ u, double* __restrict__ res, const cpfem_sell_t L,
@@ -547,6 +704,37 @@ int cpfem_elem_assemble_ex(int32_t num_cells, const int32_t* cells, const double
   }
   CPFEM_CUDA_TRY(cudaGetLastError());
   return CPFEM_OK;
+}
+
+int cpfem_node_assemble(int32_t num_cells, int32_t num_nodes, const int32_t* node_ptr, const int32_t* node_cells,
+                        const double* shape_grads, const cpfem_sell_t* sell, const uint8_t* elem_pos,
+                        const double* pk1_w, const void* tangent_w, double* residual, double* values,
+                        int32_t k_precision, void* stream) {
+  if (num_cells == 0 || num_nodes == 0) return CPFEM_OK;
+  CPFEM_REQUIRE(num_cells > 0 && num_nodes > 0 && node_ptr && node_cells && shape_grads && pk1_w,
+                "bad node assembly arguments");
+  CPFEM_REQUIRE((values == nullptr) == (tangent_w == nullptr), "values and tangent_w go together");
+  CPFEM_REQUIRE(values == nullptr || (sell && sell->group_off && sell->group_width && elem_pos),
+                "values need the layout");
+  CPFEM_REQUIRE(k_precision >= 0 && k_precision <= 2,
+                "k_precision must be 0 (FP64), 1 (FP32 stiffness) or 2 (FP32 tangent and stiffness)");
+  cudaStream_t s = (cudaStream_t)stream;
+  const int64_t G = 8 * (int64_t)num_cells;
+  const int64_t* goff = (values != nullptr) ? sell->group_off : nullptr;
+  const int32_t* gwidth = (values != nullptr) ? sell->group_width : nullptr;
+  auto run = [&](auto* kernel, auto tangent, size_t smem) -> int {
+    CPFEM_CUDA_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<(unsigned)ceil_div(num_nodes, kBlockNodes), kNodeThreads * kBlockNodes, smem, s>>>(
+        num_nodes, node_ptr, node_cells, G, shape_grads, goff, gwidth, elem_pos, pk1_w, tangent, residual, values);
+    CPFEM_CUDA_TRY(cudaGetLastError());
+    return CPFEM_OK;
+  };
+  const size_t sm32 = sizeof(NodeShared<float>) * kBlockNodes, sm64 = sizeof(NodeShared<double>) * kBlockNodes;
+  const double* t64 = static_cast<const double*>(tangent_w);
+  if (values == nullptr) return run(k_node_assemble<false, double, double>, (const double*)nullptr, 0);
+  if (k_precision == 0) return run(k_node_assemble<true, double, double>, t64, sm64);
+  if (k_precision == 1) return run(k_node_assemble<true, float, double>, t64, sm32);
+  return run(k_node_assemble<true, float, float>, static_cast<const float*>(tangent_w), sm32);
 }
 
 int cpfem_apply_dirichlet(int32_t num_bc, const int32_t* bc_dofs, const double* bc_vals, const double* u,

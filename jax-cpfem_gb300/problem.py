@@ -274,15 +274,13 @@ class CrystalPlasticity:
                                                      ("group_off", "group_width", "cols", "tpos", "diag_slot")))
         self.elem_pos = torch.tensor(epos, device=dev)
         self._csr_map = None
-        # colours of a deterministic scatter (cells of one colour share no node)
-        color = np.zeros(self.num_cells, dtype=np.int32)
-        nc = np.zeros(1, dtype=np.int32)
-        _capi.check(self.lib.cpfem_color_cells(self.num_cells, cells.ctypes.data, self.num_nodes,
-                                               color.ctypes.data, nc.ctypes.data))
-        order = np.argsort(color, kind="stable").astype(np.int32)
-        counts = np.bincount(color, minlength=int(nc[0]))
-        self.color_cells = torch.tensor(order, device=dev)
-        self.color_ptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+        # the cells of each node, for the scatter gathered by node: entries 8*cell + local node
+        flat = cells.reshape(-1)
+        ptr = np.concatenate([[0], np.cumsum(np.bincount(flat, minlength=self.num_nodes))]).astype(np.int32)
+        if np.diff(ptr).max(initial=0) > 64:
+            raise RuntimeError("more than 64 cells share a node")
+        self._node_cells = torch.tensor(np.argsort(flat, kind="stable").astype(np.int32), device=dev)
+        self._node_ptr = torch.tensor(ptr, device=dev)
 
     def _coarse_layout(self, dims):
         """Node-block pattern and sliced-ELL layout of a structured box of nodes ``dims``
@@ -783,19 +781,15 @@ class CrystalPlasticity:
                 "slip_new": torch.empty((N, G), dtype=torch.float64, device=self.device)}
 
     def scatter(self, pw, dw, res, values):
-        """Element residual / tangent scatter, colour by colour (no atomics, fixed order);
-        the element stiffness in FP32 when the problem forms its tangent in FP32."""
-        fe = self.fes[0]
-        base = self.color_cells.data_ptr()
+        """Element residual / tangent scatter, gathered by node (no atomics, fixed order), added
+        to ``res`` and ``values``; the element stiffness in FP32 when the problem forms its
+        tangent in FP32."""
         kp = 0 if values is None else (2 if dw.dtype == torch.float32 else (1 if self.fp32_tangent else 0))
         with self.region("elem_assemble"):
-            for c in range(len(self.color_ptr) - 1):
-                c0, c1 = int(self.color_ptr[c]), int(self.color_ptr[c + 1])
-                _capi.check(self.lib.cpfem_elem_assemble_ex(self.num_cells, _dev_ptr(fe.cells),
-                                                            _dev_ptr(fe.shape_grads), self.sell,
-                                                            _dev_ptr(self.elem_pos), base + 4 * c0, c1 - c0,
-                                                            _dev_ptr(pw), _dev_ptr(dw), _dev_ptr(res),
-                                                            _dev_ptr(values), kp, _stream()))
+            _capi.check(self.lib.cpfem_node_assemble(self.num_cells, self.num_nodes, _dev_ptr(self._node_ptr),
+                                                     _dev_ptr(self._node_cells), _dev_ptr(self.fes[0].shape_grads),
+                                                     self.sell, _dev_ptr(self.elem_pos), _dev_ptr(pw), _dev_ptr(dw),
+                                                     _dev_ptr(res), _dev_ptr(values), kp, _stream()))
 
     def apply_dirichlet(self, res, u, values=None):
         fe = self.fes[0]
