@@ -136,8 +136,10 @@ __global__ void __launch_bounds__(kGpThreads) k_gp_eval(const __grid_constant__ 
     cc.C44 = a.elastic_table[3 * pi + 2];
   }
 
+#pragma unroll      // the loads together (a lone warp would wait for each), the divisions in a loop
+  for (int s = 0; s < NS; ++s) Slab::kk(s) = a.g[s * G + gp];
 #pragma unroll 1
-  for (int s = 0; s < NS; ++s) Slab::ig(s) = 1.0 / a.g[s * G + gp];
+  for (int s = 0; s < NS; ++s) Slab::ig(s) = 1.0 / Slab::kk(s);
   double A[9], AR[9], Ct[9];
   mm3(F, Fpi, A);
   mm3(A, R, AR);
@@ -202,7 +204,7 @@ __global__ void __launch_bounds__(kGpThreads) k_gp_eval(const __grid_constant__ 
     for (int c = 0; c < 9; ++c) a.fpi_new[c * G + gp] = Fn[c];
   }
   if (a.slip_new != nullptr)
-#pragma unroll 2
+#pragma unroll
     for (int s = 0; s < NS; ++s) a.slip_new[s * G + gp] = a.slip[s * G + gp] + Slab::dg(s);
   if (a.g_new != nullptr)
     cp_hardening<NS, kGpThreads>(m, hh, t_sat, gss_a, rq, [&](int s) { return a.g[s * G + gp]; },

@@ -167,6 +167,17 @@ CPFEM_HD double cp_fma(double a, double b, double c) { return fma(a, b, c); }
 CPFEM_HD float cp_fma(float a, float b, float c) { return fmaf(a, b, c); }
 CPFEM_HD double cp_abs(double a) { return fabs(a); }
 CPFEM_HD float cp_abs(float a) { return fabsf(a); }
+// a > b for a, b >= 0 (or NaN: false).  An FP64 comparison takes the FP64 pipe's 64 cycles per
+// warp; the bit patterns of non-negative doubles are in the same order.
+CPFEM_HD bool cp_greater(double a, double b) {
+#ifdef __CUDA_ARCH__
+  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+  return x > y && x <= 0x7FF0000000000000LL;
+#else
+  return a > b;
+#endif
+}
+CPFEM_HD bool cp_greater(float a, float b) { return a > b; }
 
 // FP64 <-> FP32 by integer operations on the bit patterns.  GB300 issues the conversion
 // instructions on its FP64 pipe at the DFMA rate; these run on the integer pipes
@@ -226,7 +237,7 @@ CPFEM_HD void lu_factor(T* A, int* perm, T* dinv) {
 #pragma unroll
     for (int i = k + 1; i < n; ++i) {
       const T v = cp_abs(A[i * n + k]);
-      if (v > best) { best = v; p = i; }
+      if (cp_greater(v, best)) { best = v; p = i; }
     }
 #pragma unroll
     for (int i = k + 1; i < n; ++i) {

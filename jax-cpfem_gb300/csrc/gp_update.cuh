@@ -20,8 +20,8 @@
 // in shared memory, one column per thread (GpSlab), where a dynamic index costs nothing.
 // Unrolling by 2 measured best: by 1 +1 %, by 4 +7 to 17 %; three blocks per SM instead of
 // two -1 to +2 %.  Tangent passes at 262,144 points, 12 systems: 7.0 ms before the FP32
-// pre-solve and the rolling (first passes of a load step), 5.1 with the former alone, 3.3 with
-// both; later passes 2.2, 2.2 and 1.3 ms.
+// pre-solve and the rolling (first passes of a load step), 5.1 with the former alone, 3.2 now;
+// later passes 2.2, 2.2 and 1.2 ms.
 #pragma once
 
 #include "cpfem_common.cuh"
@@ -121,7 +121,7 @@ __device__ __forceinline__ void cp_residual(const MatDev& m, const Cub& cc, cons
     const double ax = fabs(x);
     // |x|^(p-1): dg = cdt |x|^(p-1) x = cdt |x|^p sign(tau) (g > 0), and the derivative
     // p cdt |x|^(p-1) / g uses the same power.
-    const double pw1 = (ax > 0.0) ? powe(ax, pexp - 1.0, ie1) : 0.0;
+    const double pw1 = cp_greater(ax, 0.0) ? powe(ax, pexp - 1.0, ie1) : 0.0;
     const double d = cdt * pw1 * x;
     const double kk = cdt * pexp * pw1 * ig;
     Slab::dg(a) = d;
@@ -175,9 +175,10 @@ __device__ __forceinline__ CubT<T> cub_of(const Cub& c) {
 }
 template <typename T>
 __device__ __forceinline__ void cubic_apply(const CubT<T>& m, const T* e, T* t) {
-  t[0] = cp_fma(m.C11, e[0], m.C12 * (e[1] + e[2]));
-  t[1] = cp_fma(m.C11, e[1], m.C12 * (e[0] + e[2]));
-  t[2] = cp_fma(m.C11, e[2], m.C12 * (e[0] + e[1]));
+  const T d = m.C11 - m.C12, p = m.C12 * (e[0] + e[1] + e[2]);
+  t[0] = cp_fma(d, e[0], p);
+  t[1] = cp_fma(d, e[1], p);
+  t[2] = cp_fma(d, e[2], p);
   t[3] = m.c44x2 * e[3];
   t[4] = m.c44x2 * e[4];
   t[5] = m.c44x2 * e[5];
@@ -186,7 +187,10 @@ __device__ __forceinline__ void cubic_apply(const CubT<T>& m, const T* e, T* t) 
 // J = dr/ds = I + sum_a kk_a (C : sym(M^T d_a (x) n_a)) (x) pv_a
 //           = I + C : Q,   Q = sum_a sym(M^T d_a (x) n_a) (x) (kk_a pv_a)
 // (C is linear, so it is applied once to the six columns of Q instead of once per slip
-// system).  In FP64, or in FP32 for a Newton direction or a tangent that need not be exact.
+// system; kk_a scales M^T d_a, and the 1/2 of sym's shear rows is in C's factor).  With the
+// comparisons of the slip powers, the scale test and the pivot search taken off the FP64 pipe,
+// that is 100 of some 1,400 FP64 instructions of an iteration: 5 % of the pass.  In FP64, or
+// in FP32 for a Newton direction or a tangent that need not be exact.
 template <int NS, int TH, typename T>
 __device__ __forceinline__ void cp_jacobian(const MatDev& m, const CubT<T>& cc, const T* M, T* J) {
   T* Q = J;   // Q accumulates in J, then J = I + C : Q column by column in place
@@ -194,6 +198,7 @@ __device__ __forceinline__ void cp_jacobian(const MatDev& m, const CubT<T>& cc, 
   for (int i = 0; i < 36; ++i) Q[i] = T(0);
 #pragma unroll 2
   for (int a = 0; a < NS; ++a) {
+    const T ka = slab_kk<NS, TH>(T(0), a);
     T d[3], n[3], w[3];
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -201,29 +206,29 @@ __device__ __forceinline__ void cp_jacobian(const MatDev& m, const CubT<T>& cc, 
       n[i] = tab_n(m, T(0), a, i);
     }
 #pragma unroll
-    for (int i = 0; i < 3; ++i) w[i] = cp_fma(M[i], d[0], cp_fma(M[3 + i], d[1], M[6 + i] * d[2]));
-    T q[6];
+    for (int i = 0; i < 3; ++i) w[i] = ka * cp_fma(M[i], d[0], cp_fma(M[3 + i], d[1], M[6 + i] * d[2]));
+    T q[6];              // rows 3 to 5 without their factor 1/2
     q[0] = w[0] * n[0];
     q[1] = w[1] * n[1];
     q[2] = w[2] * n[2];
-    q[3] = T(0.5) * cp_fma(w[1], n[2], w[2] * n[1]);
-    q[4] = T(0.5) * cp_fma(w[0], n[2], w[2] * n[0]);
-    q[5] = T(0.5) * cp_fma(w[0], n[1], w[1] * n[0]);
-    const T ka = slab_kk<NS, TH>(T(0), a);
+    q[3] = cp_fma(w[1], n[2], w[2] * n[1]);
+    q[4] = cp_fma(w[0], n[2], w[2] * n[0]);
+    q[5] = cp_fma(w[0], n[1], w[1] * n[0]);
     T c[6];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) c[j] = ka * tab_pv(m, T(0), a, j);
+    for (int j = 0; j < 6; ++j) c[j] = tab_pv(m, T(0), a, j);
 #pragma unroll
     for (int i = 0; i < 6; ++i)
 #pragma unroll
       for (int j = 0; j < 6; ++j) Q[6 * i + j] = cp_fma(q[i], c[j], Q[6 * i + j]);
   }
+  const CubT<T> ch{cc.C11, cc.C12, T(0.5) * cc.c44x2};
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
     T col[6], t[6];
 #pragma unroll
     for (int i = 0; i < 6; ++i) col[i] = Q[6 * i + j];
-    cubic_apply(cc, col, t);
+    cubic_apply(ch, col, t);
 #pragma unroll
     for (int i = 0; i < 6; ++i) J[6 * i + j] = (i == j ? T(1) : T(0)) + t[i];
   }
@@ -235,14 +240,14 @@ constexpr double kJ32Scale = 1e4;
 
 template <int NS, int TH>
 __device__ __forceinline__ bool scale_f32_ok(const Cub& cc) {
-  double kmax = 0.0;
+  float kmax = 0.0f;
 #pragma unroll 2
-  for (int a = 0; a < NS; ++a) kmax = fmax(kmax, GpSlab<NS, TH>::kk(a));
-  return kmax * cc.C11 <= kJ32Scale;
+  for (int a = 0; a < NS; ++a) kmax = fmaxf(kmax, GpSlab<NS, TH>::kf(a));
+  return kmax * f32_of(cc.C11) <= (float)kJ32Scale;
 }
 
-// A Newton direction ds = -J^-1 r at the slab's derivatives.  Out of line: one copy of the code
-// serves the local solve and the FP32 pre-solve.
+// A Newton direction ds = -J^-1 r at the slab's derivatives.  (Out of line it measured 1 %
+// slower on few points and 1 % faster on the first passes of 262,144.)
 template <typename T>
 struct DirIn {
   T M[9], r[6];
@@ -253,7 +258,7 @@ struct Vec6 {
   T v[6];
 };
 template <int NS, int TH, typename T>
-__device__ __noinline__ Vec6<T> cp_direction(const MatDev& m, DirIn<T> in) {
+__device__ __forceinline__ Vec6<T> cp_direction(const MatDev& m, DirIn<T> in) {
   T J[36], dinv[6];
   int perm[6];
   cp_jacobian<NS, TH, T>(m, in.cc, in.M, J);
@@ -659,9 +664,8 @@ __device__ __forceinline__ void cp_hardening(const MatDev& m, double h, double t
   for (int b = 0; b < NS; ++b) {
     const double ratio = 1.0 - old_g(b) / t_sat;
     const double ar = fabs(ratio);
-    const double pw = (ar > 0.0) ? powe(ar, gss_a, ia) : 0.0;
-    const double sg = (ratio > 0.0) ? 1.0 : ((ratio < 0.0) ? -1.0 : 0.0);
-    const double t = h * fabs(Slab::dg(b)) * pw * sg;
+    const double pw = cp_greater(ar, 0.0) ? powe(ar, gss_a, ia) : 0.0;
+    const double t = h * fabs(Slab::dg(b)) * copysign(pw, ratio);     // pw = 0 where ratio is 0 or NaN
     Slab::ig(b) = t;
     total += t;
   }
