@@ -762,15 +762,15 @@ def main():
                    "traffic": KRYLOV_DRAM_BYTES_PER_LAUNCH.get(kr_key) if n == N_EDGE else None,
                    "traffic_note": "DRAM bytes per launch (ncu); algorithmic bytes per launch = "
                                    "algorithmic_bytes_per_iteration x iterations, served from L2",
-                   "kernel": ("k_bicgstab<0,%d> (persistent multigrid-preconditioned BiCGSTAB, %s V-cycle, one "
-                              "launch per linear solve)" % ((2, "FP32") if mg_fp32 else (1, "FP64"))
+                   "kernel": ("k_bicgstab_team (persistent multigrid-preconditioned BiCGSTAB, %s V-cycle, one "
+                              "launch per linear solve)" % ("FP32" if mg_fp32 else "FP64")
                               if args.precond == 3 else
-                              "k_bicgstab<0,0> (persistent BiCGSTAB, one launch per linear solve)"),
+                              "k_bicgstab_team (persistent BiCGSTAB, one launch per linear solve)"),
                    "launches": kr_n, "us_per_iteration": kr_ms * 1e3 / max(kr_its, 1),
                    "algorithmic_bytes_per_iteration": kb, "flops_per_iteration": kf,
                    "fp32_flops_per_iteration": kf32,
-                   "limiter": ("grid barriers and load latency (29 grid barriers per iteration; ncu: barrier "
-                               "and long-scoreboard stalls dominate, FP64 pipe 15-17 %)" if args.precond == 3
+                   "limiter": ("grid barriers, the fine level's operator passes from L2 and the FP64 products"
+                               if args.precond == 3
                                else "FP64 pipe (the SpMVs)"),
                    "hbm": {"achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm if hbm else None},
                    "peak_source": "cpfem_probe_dfma FP64 (of measured); HBM from MEASURED_PEAKS.json (of measured)"}
@@ -873,15 +873,16 @@ def max_over_ranks(t, world, device):
 
 class CountingLib:
     """Forwards to the C ABI and counts the kernels its calls launch, from the sources:
-    cpfem_bicgstab_ex is the persistent launch, plus the point preconditioner's set-up
-    (precond 1, 2) and the two true-residual kernels (flags bit 0); cpfem_mg_setup is the
+    cpfem_bicgstab_ex is the persistent launch (a system too big for shared memory adds the
+    preconditioner's set-up and the true residual, not counted here); cpfem_mg_setup is the
     level-0 block inverses, three directional Galerkin passes and a block inversion per
-    coarse level, and two FP32 copies per level for the FP32 V-cycle; every other listed
-    entry point launches one kernel."""
+    coarse level, and for the FP32 V-cycle copies of the coarse operators and of every
+    level's inverses (the dense coarse operator, where there is one, not counted); every
+    other listed entry point launches one kernel."""
     LAUNCHES = {"cpfem_gp_eval": 1, "cpfem_elem_assemble": 1, "cpfem_elem_assemble_ex": 1, "cpfem_node_assemble": 1, "cpfem_apply_dirichlet": 1, "cpfem_dot": 1,
-                "cpfem_bc_initial_guess": 1, "cpfem_axpy": 1, "cpfem_spmv": 1, "cpfem_bicgstab": 2,
-                "cpfem_bicgstab_ex": 2, "cpfem_cell_average": 1, "cpfem_segmented_dot": 1,
-                "cpfem_bicgstab_batched": 2, "cpfem_gp_vjp": 1}
+                "cpfem_bc_initial_guess": 1, "cpfem_axpy": 1, "cpfem_spmv": 1, "cpfem_bicgstab": 1,
+                "cpfem_bicgstab_ex": 1, "cpfem_cell_average": 1, "cpfem_segmented_dot": 1,
+                "cpfem_bicgstab_batched": 1, "cpfem_gp_vjp": 1}
 
     def __init__(self, lib):
         self._lib = lib
@@ -890,12 +891,9 @@ class CountingLib:
 
     @staticmethod
     def _count(name, a, k):
-        if name == "cpfem_bicgstab_ex":
-            o = a[4]._obj
-            return 1 + (1 if o.precond in (1, 2) else 0) + (2 if o.flags & 1 else 0)
         if name == "cpfem_mg_setup":
             mg = a[0]._obj
-            return 1 + 4 * (mg.num_levels - 1) + (2 * mg.num_levels if mg.precision == 1 else 0)
+            return 1 + 4 * (mg.num_levels - 1) + (2 * mg.num_levels - 1 if mg.precision == 1 else 0)
         return k
 
     def __getattr__(self, name):

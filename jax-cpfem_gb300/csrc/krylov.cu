@@ -5,8 +5,10 @@
 // three rows without any cross-lane reduction -- on GB300 the FP64 pipe, not HBM, is
 // the SpMV's limit, and a shuffle reduction would cost as many FP64 adds as the FMAs.
 //
-// BiCGSTAB runs as one cooperative launch: every block owns a fixed set of nodes, the
-// five global dependencies of an iteration (the halo of phat and shat, four dot
+// BiCGSTAB runs as one cooperative launch.  Systems whose vectors fit the blocks' shared
+// memory, and every multigrid solve, use the kernel of krylov_team.cuh; the kernels here
+// stream their vectors from memory, for larger systems and for batches of many.  In them
+// every block owns a fixed set of nodes, the five global dependencies of an iteration (the halo of phat and shat, four dot
 // products) are crossed with a grid barrier, and every block reduces the per-block
 // partial sums in the same fixed order, so all blocks hold bitwise-identical scalars
 // and take the same branch.  Barrier waits are bounded: a block that waits too long sets
