@@ -153,16 +153,6 @@ CPFEM_HD void cubic_apply(const Cub& m, const double* e, double* t) {
   t[5] = c2 * e[5];
 }
 
-CPFEM_HD void cubic_apply(const Cub& m, const float* e, float* t) {
-  const float c11 = (float)m.C11, c12 = (float)m.C12, c2 = (float)(2.0 * m.C44);
-  t[0] = fmaf(c11, e[0], c12 * (e[1] + e[2]));
-  t[1] = fmaf(c11, e[1], c12 * (e[0] + e[2]));
-  t[2] = fmaf(c11, e[2], c12 * (e[0] + e[1]));
-  t[3] = c2 * e[3];
-  t[4] = c2 * e[4];
-  t[5] = c2 * e[5];
-}
-
 CPFEM_HD double cp_fma(double a, double b, double c) { return fma(a, b, c); }
 CPFEM_HD float cp_fma(float a, float b, float c) { return fmaf(a, b, c); }
 CPFEM_HD double cp_abs(double a) { return fabs(a); }
