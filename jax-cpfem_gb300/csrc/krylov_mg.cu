@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(512, 1) k_mg_dense(const cpfem_mg_t mg, int lb
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     MgTag t{kMgTagMagic, (const void*)A.minv(lb), lb, (int)mg.sell[lb].num_nodes, (int)sizeof(R), 0};
-    *mg_tag<R>(mg, lb) = t;
+    *mg_tag(mg) = t;
   }
 }
 

@@ -294,6 +294,19 @@ __device__ __forceinline__ void mg_prolong(const cpfem_mg_t& mg, int l, R* X, co
 
 constexpr int kMgDenseNodes = 256;   // largest level that becomes a dense operator
 
+// What the dense operator in scratch[0] belongs to: written in front of it by the set-up, checked
+// by a solve, which smooths the levels itself where it does not match.  The Galerkin passes of
+// every set-up write scratch[0] from its first element on, so a set-up of any size that uses the
+// same scratch, one that forms no dense operator too, takes the tag of the one before away.
+struct MgTag {
+  unsigned long long magic;
+  const void* minv;
+  int level, nodes, real_bytes, pad;
+};
+constexpr unsigned long long kMgTagMagic = 0x6D67636F61727365ull;
+constexpr size_t kMgTagBytes = 64;
+static_assert(sizeof(MgTag) <= kMgTagBytes, "the tag fits in front of the operator");
+
 // The first level of the dense part (num_levels: none): the coarsest levels, from level 1 on,
 // with at most local_nodes (0: 256, and never more than 256) nodes, whose operator and tag fit
 // in scratch[0].
@@ -302,28 +315,17 @@ __host__ __device__ inline int mg_dense_level(const cpfem_mg_t& mg, size_t real_
   int lb = mg.num_levels;
   for (int l = mg.num_levels - 1; l >= 1 && mg.sell[l].num_nodes <= most; --l) {
     const size_t n = 3 * (size_t)mg.sell[l].num_nodes;
-    if (n * n * real_bytes + 64 > sizeof(double) * 243 * (size_t)mg.scratch_nodes) break;
+    if (n * n * real_bytes + kMgTagBytes > sizeof(double) * 243 * (size_t)mg.scratch_nodes) break;
     lb = l;
   }
   return lb;
 }
 
-// What the dense operator in scratch[0] belongs to: written behind it by the set-up, checked by
-// a solve, which smooths the levels itself where it does not match.
-struct MgTag {
-  unsigned long long magic;
-  const void* minv;
-  int level, nodes, real_bytes, pad;
-};
-constexpr unsigned long long kMgTagMagic = 0x6D67636F61727365ull;
-
 template <typename R>
-__host__ __device__ inline R* mg_dense(const cpfem_mg_t& mg) { return reinterpret_cast<R*>(mg.scratch[0]); }
-template <typename R>
-__host__ __device__ inline MgTag* mg_tag(const cpfem_mg_t& mg, int lb) {
-  const size_t n = 3 * (size_t)mg.sell[lb].num_nodes;
-  return reinterpret_cast<MgTag*>(reinterpret_cast<char*>(mg.scratch[0]) + ((n * n * sizeof(R) + 15) / 16) * 16);
+__host__ __device__ inline R* mg_dense(const cpfem_mg_t& mg) {
+  return reinterpret_cast<R*>(reinterpret_cast<char*>(mg.scratch[0]) + kMgTagBytes);
 }
+__host__ __device__ inline MgTag* mg_tag(const cpfem_mg_t& mg) { return reinterpret_cast<MgTag*>(mg.scratch[0]); }
 
 constexpr size_t kMgStageBytes = 220 * 1024;    // shared memory of a dense set-up's block, at most
 
@@ -463,7 +465,7 @@ __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg,
   const int64_t tq = 8 * ((int64_t)wid * tm.nb + rank) + (lane >> 2), sq = 8 * (int64_t)warps * tm.nb;
   int lb = mg_dense_level(mg, sizeof(R));
   if (lb < L) {
-    const MgTag* tag = mg_tag<R>(mg, lb);
+    const MgTag* tag = mg_tag(mg);
     if (tag->magic != kMgTagMagic || tag->minv != (const void*)A.minv(lb) || tag->level != lb ||
         tag->nodes != mg.sell[lb].num_nodes || tag->real_bytes != (int)sizeof(R))
       lb = L;

@@ -1,0 +1,37 @@
+"""What a multigrid set-up leaves for the solves that follow it: whose dense coarse operator lies in
+the hierarchy's scratch, and the settings it was formed with."""
+import pytest
+import torch
+
+from tests.test_gpu_point_solver import _residual, _system
+
+pytestmark = pytest.mark.gpu
+
+
+def _kept(prob):
+    """The problem's next solves use its hierarchy as it stands."""
+    prob.mg_setup = lambda *a, **kw: prob._mg
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("local_nodes", [256, 1])
+def test_smaller_hierarchy_in_the_same_scratch(pkg, gpu, precision, local_nodes):
+    """A 4^3 hierarchy set up in a 16^3 one's scratch writes the front of it only (with a dense
+    operator of its own or, local_nodes = 1, without): the 16^3 solve finds that, smooths its
+    coarse levels itself, and is bit for bit the solve that was told to (local_nodes = 1)."""
+    problem_mod, solver_mod = gpu
+    p1, A1, b1, x1 = _system(pkg, problem_mod, solver_mod, (16, 16, 16))
+    p2, A2, b2, x2 = _system(pkg, problem_mod, solver_mod, (4, 4, 4))
+    p1.mg_setup(A1.values, precision=precision)
+    _kept(p1)
+    solve = lambda: solver_mod.bicgstab(p1, A1, b1, x1, precond=3, atol=1e-30, maxiter=200)
+    dense, k0, ok = solve()
+    assert ok
+    m2 = p2.multigrid(precision=precision, local_nodes=local_nodes)
+    m2.scratch[0], m2.scratch[1] = p1._mg.scratch[0], p1._mg.scratch[1]
+    p2.mg_setup(A2.values, precision=precision, local_nodes=local_nodes)
+    x, k, ok = solve()
+    p1._mg.local_nodes = 1
+    ref, kr, _ = solve()
+    assert ok and k == kr and torch.equal(x, ref)
+    assert abs(k - k0) <= 2 and _residual(A1, x, b1) <= 2e-10 * float(b1.norm())
