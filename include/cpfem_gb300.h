@@ -400,7 +400,9 @@ typedef struct {
                                                  [243*scratch_nodes].  scratch[0] then holds the small
                                                  coarse levels' part of the cycle as a dense operator
                                                  until the next set-up (a solve that finds another
-                                                 hierarchy's there smooths the levels itself) */
+                                                 hierarchy's there, or one formed with other sweep
+                                                 counts, omega or local_nodes than its own, smooths
+                                                 the levels itself) */
   int64_t scratch_nodes;                      /* >= max over l of dims_c[0]*dims[l][1]*dims[l][2] */
   int32_t precision;       /* 0: the V-cycle in FP64 on the arrays above; 1: in FP32 on the
                               arrays below (set up from the FP64 operators).  The Krylov

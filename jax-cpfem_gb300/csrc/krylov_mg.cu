@@ -142,10 +142,7 @@ __global__ void __launch_bounds__(512, 1) k_mg_dense(const cpfem_mg_t mg, int lb
     for (int i = threadIdx.x; i < N; i += blockDim.x) K[(size_t)i * N + c] = X[i];
     __syncthreads();
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    MgTag t{kMgTagMagic, (const void*)A.minv(lb), lb, (int)mg.sell[lb].num_nodes, (int)sizeof(R), 0};
-    *mg_tag(mg) = t;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *mg_tag(mg) = mg_tag_of<R>(mg, A.minv(lb), lb);
 }
 
 template <typename R>

@@ -294,14 +294,17 @@ __device__ __forceinline__ void mg_prolong(const cpfem_mg_t& mg, int l, R* X, co
 
 constexpr int kMgDenseNodes = 256;   // largest level that becomes a dense operator
 
-// What the dense operator in scratch[0] belongs to: written in front of it by the set-up, checked
-// by a solve, which smooths the levels itself where it does not match.  The Galerkin passes of
+// What the dense operator in scratch[0] belongs to and was formed with: written in front of it by
+// the set-up, checked by a solve, which smooths the levels itself where it does not match (the
+// smoother's settings may change between set-up and solve: those levels then follow them as the
+// others do).  The Galerkin passes of
 // every set-up write scratch[0] from its first element on, so a set-up of any size that uses the
 // same scratch, one that forms no dense operator too, takes the tag of the one before away.
 struct MgTag {
   unsigned long long magic;
   const void* minv;
-  int level, nodes, real_bytes, pad;
+  long long omega;       // its bits
+  int levels, level, nodes, real_bytes, pre_sweeps, post_sweeps, coarse_sweeps, pad;
 };
 constexpr unsigned long long kMgTagMagic = 0x6D67636F61727365ull;
 constexpr size_t kMgTagBytes = 64;
@@ -326,6 +329,16 @@ __host__ __device__ inline R* mg_dense(const cpfem_mg_t& mg) {
   return reinterpret_cast<R*>(reinterpret_cast<char*>(mg.scratch[0]) + kMgTagBytes);
 }
 __host__ __device__ inline MgTag* mg_tag(const cpfem_mg_t& mg) { return reinterpret_cast<MgTag*>(mg.scratch[0]); }
+template <typename R>
+__device__ __forceinline__ MgTag mg_tag_of(const cpfem_mg_t& mg, const R* minv, int lb) {
+  return MgTag{kMgTagMagic, minv, __double_as_longlong(mg.omega), mg.num_levels, lb, (int)mg.sell[lb].num_nodes, (int)sizeof(R),
+               mg.pre_sweeps, mg.post_sweeps, mg.coarse_sweeps, 0};
+}
+__device__ __forceinline__ bool mg_tag_same(const MgTag& a, const MgTag& b) {
+  return a.magic == b.magic && a.minv == b.minv && a.omega == b.omega && a.levels == b.levels && a.level == b.level &&
+         a.nodes == b.nodes && a.real_bytes == b.real_bytes && a.pre_sweeps == b.pre_sweeps &&
+         a.post_sweeps == b.post_sweeps && a.coarse_sweeps == b.coarse_sweeps;
+}
 
 constexpr size_t kMgStageBytes = 220 * 1024;    // shared memory of a dense set-up's block, at most
 
@@ -464,12 +477,7 @@ __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg,
   const int q = lane & 3;
   const int64_t tq = 8 * ((int64_t)wid * tm.nb + rank) + (lane >> 2), sq = 8 * (int64_t)warps * tm.nb;
   int lb = mg_dense_level(mg, sizeof(R));
-  if (lb < L) {
-    const MgTag* tag = mg_tag(mg);
-    if (tag->magic != kMgTagMagic || tag->minv != (const void*)A.minv(lb) || tag->level != lb ||
-        tag->nodes != mg.sell[lb].num_nodes || tag->real_bytes != (int)sizeof(R))
-      lb = L;
-  }
+  if (lb < L && !mg_tag_same(*mg_tag(mg), mg_tag_of<R>(mg, A.minv(lb), lb))) lb = L;
   auto barrier = [&]() { pt_reduce<0>(nullptr, 0, tm, a, sh); };
   const R* Mi0 = A.minv(0);
   // one sweep of level 0 after its row sums: f(node, X + om D^-1 (v - A X))

@@ -321,7 +321,9 @@ class CrystalPlasticity:
         operators (the Krylov iteration and its stop rule stay FP64): faster, but not for
         near-singular systems, where ``solver.bicgstab`` falls back to FP64 by itself.
         Coarse levels with at most ``local_nodes`` nodes (256 at most) are applied as one dense
-        operator, formed by ``mg_setup`` with the sweep counts it is given."""
+        operator, formed by ``mg_setup`` with the sweep counts and damping it is given; a solve
+        with others (``refresh="step"`` keeps the set-up) smooths those levels until the next
+        set-up."""
         if precision not in ("fp64", "fp32"):
             raise ValueError("multigrid precision must be 'fp64' or 'fp32'")
         if getattr(self, "_mg", None) is not None and self._mg_key == max_levels:

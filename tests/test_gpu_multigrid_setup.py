@@ -35,3 +35,20 @@ def test_smaller_hierarchy_in_the_same_scratch(pkg, gpu, precision, local_nodes)
     ref, kr, _ = solve()
     assert ok and k == kr and torch.equal(x, ref)
     assert abs(k - k0) <= 2 and _residual(A1, x, b1) <= 2e-10 * float(b1.norm())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("change", [{"coarse_sweeps": 9}, {"pre_sweeps": 2}, {"post_sweeps": 2}, {"omega": 0.3}, {}])
+def test_settings_changed_under_a_kept_set_up(pkg, gpu, precision, change):
+    """refresh="step" keeps the set-up while the smoother's settings change: the solve is bit for
+    bit the one that smooths every level with the new settings (local_nodes = 1).  Unchanged
+    settings use the dense operator, whose rounding differs."""
+    problem_mod, solver_mod = gpu
+    prob, A, b, x0 = _system(pkg, problem_mod, solver_mod, (8, 8, 8))
+    prob.mg_setup(A.values, precision=precision, pre_sweeps=1, post_sweeps=1, coarse_sweeps=4, omega=0.45)
+    opts = {"precision": precision, "refresh": "step", **change}
+    solve = lambda **kw: solver_mod.bicgstab(prob, A, b, x0, precond=3, atol=1e-30, mg_options={**opts, **kw})
+    x, k, ok = solve()
+    ref, kr, _ = solve(local_nodes=1)
+    assert ok and _residual(A, x, b) <= 2e-10 * float(b.norm())
+    assert torch.equal(x, ref) == bool(change) and abs(k - kr) <= (0 if change else 2)
