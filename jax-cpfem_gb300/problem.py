@@ -388,7 +388,7 @@ class CrystalPlasticity:
         mg.scratch[0], mg.scratch[1] = buf(243 * sn), buf(243 * sn)
         mg.scratch_nodes = sn
         self._mg, self._mg_keep, self._mg_free, self._mg_key = mg, keep, free, max_levels
-        self._mg_bc_token = None
+        self._mg_bc_token = self._mg_setup_key = None     # nothing of an earlier hierarchy's set-up holds
         self.mg_levels = levels
         mg.local_nodes = int(local_nodes)
         self._mg_precision(mg, precision)

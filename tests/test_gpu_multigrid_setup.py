@@ -52,3 +52,14 @@ def test_settings_changed_under_a_kept_set_up(pkg, gpu, precision, change):
     ref, kr, _ = solve(local_nodes=1)
     assert ok and _residual(A, x, b) <= 2e-10 * float(b.norm())
     assert torch.equal(x, ref) == bool(change) and abs(k - kr) <= (0 if change else 2)
+
+
+def test_other_levels_under_a_kept_set_up(pkg, gpu):
+    """max_levels makes a new hierarchy: it is set up although refresh="step" found the step's key."""
+    problem_mod, solver_mod = gpu
+    prob, A, b, x0 = _system(pkg, problem_mod, solver_mod, (8, 8, 8))
+    prob.mg_setup(A.values, refresh="step")
+    x, k, ok = solver_mod.bicgstab(prob, A, b, x0, precond=3, atol=1e-30, maxiter=200,
+                                   mg_options={"refresh": "step", "max_levels": 2})
+    ref, kr, _ = solver_mod.bicgstab(prob, A, b, x0, precond=3, atol=1e-30, mg_options={"max_levels": 2})
+    assert ok and k == kr and torch.equal(x, ref)
