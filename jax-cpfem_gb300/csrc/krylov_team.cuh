@@ -174,13 +174,16 @@ __device__ __forceinline__ float opval<float>(double v) {
   return __uint_as_float(bits);
 }
 
-// a > b for a, b that are sums of squares or NaN (then false), and v == 0, without the FP64 pipe.
+// a > b, and a <= b, for a, b that are sums of squares or NaN of either sign (CUDA's own has it set;
+// then false), and v == 0, without the FP64 pipe.
+__device__ __forceinline__ long long pt_bits(double v) { return __double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFll; }
 __device__ __forceinline__ bool pt_greater(double a, double b) {
-  const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-  return x > y && x <= 0x7FF0000000000000ll && y <= 0x7FF0000000000000ll;
+  const long long x = pt_bits(a), y = pt_bits(b);
+  return x > y && x <= 0x7FF0000000000000ll;    // b NaN: no x that is none lies above it
 }
 __device__ __forceinline__ bool pt_at_most(double a, double b) {
-  return __double_as_longlong(a) <= __double_as_longlong(b);   // false for a NaN a
+  const long long x = pt_bits(a), y = pt_bits(b);
+  return x <= y && y <= 0x7FF0000000000000ll;
 }
 __device__ __forceinline__ bool pt_zero(double v) { return (__double_as_longlong(v) << 1) == 0ll; }
 

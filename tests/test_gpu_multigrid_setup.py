@@ -63,3 +63,17 @@ def test_other_levels_under_a_kept_set_up(pkg, gpu):
                                    mg_options={"refresh": "step", "max_levels": 2})
     ref, kr, _ = solver_mod.bicgstab(prob, A, b, x0, precond=3, atol=1e-30, mg_options={"max_levels": 2})
     assert ok and k == kr and torch.equal(x, ref)
+
+
+@pytest.mark.parametrize("bits", [0x7FC00000, -0x400000])       # a NaN without, and with its sign bit
+def test_fp32_cycle_that_goes_to_nan_reports_it(pkg, gpu, bits, monkeypatch):
+    """Code -12 whatever the NaN's sign (the FP32 diagonal blocks of level 0 are overwritten)."""
+    problem_mod, solver_mod = gpu
+    prob, A, b, x0 = _system(pkg, problem_mod, solver_mod, (4, 4, 4))
+    prob.mg_setup(A.values, precision="fp32")
+    minv, = [t for t in prob._mg_keep if t.data_ptr() == prob._mg.minv32[0]]
+    minv.view(torch.int32).fill_(bits)
+    _kept(prob)
+    monkeypatch.setattr(solver_mod, "_fp32_solve_ok", lambda *a: True)      # no FP64 solve after it
+    x, k, ok = solver_mod.bicgstab(prob, A, b, x0, precond=3)
+    assert k == -12 and not ok
