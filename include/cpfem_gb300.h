@@ -537,6 +537,16 @@ int cpfem_bicgstab_batched(const cpfem_sell_t* sell, const double* values, const
  */
 int cpfem_probe_dfma(int64_t iters, int32_t blocks, double* out, double* flops, void* stream);
 
+/*
+ * Failure test (not on the solve path): cpfem_bicgstab_ex with waits of at most `polls` polls
+ * (1 .. 2^20, about 0.4 us each) and one arrival short at the grid barriers, as if a block were
+ * lost.  The waits run out, and the call returns CPFEM_ERR_SOLVE (or a report with its error word
+ * set), the GPU usable as before; a solve of one block that waits for none is not disturbed.
+ */
+int cpfem_probe_lost_block(const cpfem_sell_t* sell, const double* values, const double* b, double* x,
+                           const cpfem_krylov_opts_t* opts, int32_t polls, void* workspace, int32_t* info,
+                           void* stream);
+
 #ifdef __cplusplus
 }
 #endif

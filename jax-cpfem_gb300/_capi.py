@@ -209,6 +209,7 @@ SIGNATURES = {
     "cpfem_struct_size": (ctypes.c_size_t, [_I32]),
     "cpfem_mg_setup": (ctypes.c_int, [ctypes.POINTER(MGHierarchy), _P, _P]),
     "cpfem_bicgstab_ex": (ctypes.c_int, [_SP, _P, _P, _P, ctypes.POINTER(KrylovOpts), _P, _P, _P]),
+    "cpfem_probe_lost_block": (ctypes.c_int, [_SP, _P, _P, _P, ctypes.POINTER(KrylovOpts), _I32, _P, _P, _P]),
     "cpfem_bicgstab_batched_workspace_bytes": (ctypes.c_size_t, [_I32]),
     "cpfem_bicgstab_batched": (ctypes.c_int, [_SP, _P, _P, _P, _I32, _D, _D, _I32, _I32, _P, _I32, _P, _P, _P, _P, _P]),
     "cpfem_probe_dfma": (ctypes.c_int, [_I64, _I32, _P, _P, _P]),

@@ -34,7 +34,7 @@ struct GridSync {
   unsigned int count;   // arrivals so far (monotonic within a launch)
   unsigned int gen;     // unused (kept for the layout)
   int error;
-  int pad;
+  int polls;            // of a wait, at most (0: kSpinLimit)
 };
 
 // the launch's report, written by the kernel into the workspace (the public layout)
@@ -176,8 +176,9 @@ __device__ __forceinline__ void red_release_add_u32(unsigned int* p, unsigned in
 // complete when it reaches k*nb.  Thread 0 arrives with a release reduction, which
 // publishes every write the block made before the __syncthreads, and waits with acquire
 // loads; no reset is needed, so the last arrival costs no extra round trip.  The wait is
-// bounded: after kSpinLimit polls the block records an error (also in *gerr) and returns
-// false instead of hanging.
+// bounded: after kSpinLimit polls (gs->polls, where that is set) the block records an error (also
+// in *gerr) and returns false instead of hanging; on that error the others' waits and its own later
+// ones end too.
 __device__ __forceinline__ bool counted_barrier(GridSync* gs, unsigned int nb, unsigned int& gen, int* gerr) {
   __shared__ int s_ok;
   __syncthreads();
@@ -187,7 +188,7 @@ __device__ __forceinline__ bool counted_barrier(GridSync* gs, unsigned int nb, u
     red_release_add_u32(&gs->count, 1u);
     long long spins = 0;
     while (ld_acquire_u32(&gs->count) < target) {
-      if (++spins > kSpinLimit) {
+      if ((++spins & 63) == 0 && (spins >= (gs->polls > 0 ? gs->polls : kSpinLimit) || *(volatile int*)&gs->error != 0)) {
         ok = 0;
         atomicExch(&gs->error, 1);
         if (gerr != nullptr) atomicExch(gerr, 1);
@@ -464,7 +465,7 @@ template <bool TRANS>
 static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double* b, double* x, int precond,
                         double tol, double atol, int32_t maxiter, void* workspace, int32_t* info, cudaStream_t s,
                         int max_restarts = 0, const cpfem_mg_t* mgp = nullptr, int grid_blocks = 0,
-                        int flags = 0, cpfem_solve_report_t* report = nullptr) {
+                        int flags = 0, cpfem_solve_report_t* report = nullptr, int lost_polls = 0) {
   KWork w;
   carve(workspace, L.num_nodes, &w);
   PointPlan plan{};
@@ -475,14 +476,17 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
     a.phat = w.phat; a.shat = w.shat;
     a.counters = (unsigned int*)w.partials;
     a.cells = w.partials + kPointCounterBytes / sizeof(double);
-    a.error = &w.sync->error;
+    a.error = &w.out->error;
+    a.polls = lost_polls > 0 ? lost_polls : kPtSpinLimit;
     a.out = w.out;
     a.precond = precond; a.maxiter = maxiter; a.max_restarts = max_restarts;
     a.true_res = (flags & kKrylovTrueResidual) ? 1 : 0;
     a.tol = tol; a.atol = atol;
-    // one memset over the error word, the report and the one team's counter (neighbours in the
-    // workspace)
+    // one memset over the report with its error word and the one team's counter (neighbours in
+    // the workspace)
     CPFEM_CUDA_TRY(cudaMemsetAsync(w.sync, 0, (size_t)((char*)w.partials - (char*)w.sync) + 128, s));
+    // the failure test: one arrival short (the count's first increment wraps it to 0)
+    if (lost_polls > 0) CPFEM_CUDA_TRY(cudaMemsetAsync(a.counters, 0xFF, sizeof(unsigned int), s));
     if (!plan.ok) {
       double* const v[8] = {w.r, w.rhat, w.p, w.q, w.t, w.s, w.minv, w.minv + 3 * (size_t)L.num_nodes};
       std::copy(v, v + 8, a.vectors);
@@ -492,6 +496,10 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
     return finish_solve(w.out, info, flags, report, s);
   }
   CPFEM_CUDA_TRY(cudaMemsetAsync(w.sync, 0, sizeof(GridSync), s));
+  if (lost_polls > 0) {
+    const GridSync short_one = {~0u, 0u, 0, lost_polls};
+    CPFEM_CUDA_TRY(cudaMemcpyAsync(w.sync, &short_one, sizeof(short_one), cudaMemcpyHostToDevice, s));
+  }
   if (precond == 1 || precond == 2) {
     k_precond_setup<TRANS><<<(unsigned)ceil_div(L.num_nodes, 128), 128, 0, s>>>(L, vals, precond, w.minv);
     CPFEM_CUDA_TRY(cudaGetLastError());
@@ -569,8 +577,9 @@ int cpfem_bicgstab_last_stats_ex(double* out, int32_t n) {
   return CPFEM_OK;
 }
 
-int cpfem_bicgstab_ex(const cpfem_sell_t* sell, const double* values, const double* b, double* x,
-                      const cpfem_krylov_opts_t* opts, void* workspace, int32_t* info, void* stream) {
+static int solve_checked(const cpfem_sell_t* sell, const double* values, const double* b, double* x,
+                         const cpfem_krylov_opts_t* opts, void* workspace, int32_t* info, void* stream,
+                         int lost_polls) {
   CPFEM_REQUIRE(info != nullptr, "info is null");
   info[0] = 0;
   info[1] = 1;
@@ -593,9 +602,24 @@ int cpfem_bicgstab_ex(const cpfem_sell_t* sell, const double* values, const doub
   cudaStream_t s = (cudaStream_t)stream;
   if (opts->transpose)
     return run_bicgstab<true>(*sell, values, b, x, opts->precond, opts->tol, opts->atol, opts->maxiter, workspace,
-                              info, s, opts->max_restarts, opts->mg, opts->grid_blocks, opts->flags, opts->report);
+                              info, s, opts->max_restarts, opts->mg, opts->grid_blocks, opts->flags, opts->report,
+                              lost_polls);
   return run_bicgstab<false>(*sell, values, b, x, opts->precond, opts->tol, opts->atol, opts->maxiter, workspace,
-                             info, s, opts->max_restarts, opts->mg, opts->grid_blocks, opts->flags, opts->report);
+                             info, s, opts->max_restarts, opts->mg, opts->grid_blocks, opts->flags, opts->report,
+                             lost_polls);
+}
+
+int cpfem_bicgstab_ex(const cpfem_sell_t* sell, const double* values, const double* b, double* x,
+                      const cpfem_krylov_opts_t* opts, void* workspace, int32_t* info, void* stream) {
+  return solve_checked(sell, values, b, x, opts, workspace, info, stream, 0);
+}
+
+int cpfem_probe_lost_block(const cpfem_sell_t* sell, const double* values, const double* b, double* x,
+                           const cpfem_krylov_opts_t* opts, int32_t polls, void* workspace, int32_t* info,
+                           void* stream) {
+  CPFEM_REQUIRE(info != nullptr, "info is null");
+  CPFEM_REQUIRE(polls >= 1 && polls <= (1 << 20), "bad probe arguments");
+  return solve_checked(sell, values, b, x, opts, workspace, info, stream, polls);
 }
 
 int cpfem_bicgstab(const cpfem_sell_t* sell, const double* values, const double* b, double* x, int32_t precond,
@@ -995,6 +1019,7 @@ int cpfem_bicgstab_batched(const cpfem_sell_t* sell, const double* values, const
     a.counters = (unsigned int*)w.partials;
     a.cells = w.partials + kPointCounterBytes / sizeof(double);
     a.error = w.error;
+    a.polls = kPtSpinLimit;
     a.teams = (PointTeam*)w.teams;
     a.team_of_block = w.team_of_block;
     a.info = w.info;

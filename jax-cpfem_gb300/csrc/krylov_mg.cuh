@@ -335,9 +335,18 @@ __device__ __forceinline__ MgTag mg_tag_of(const cpfem_mg_t& mg, const R* minv, 
                mg.pre_sweeps, mg.post_sweeps, mg.coarse_sweeps, 0};
 }
 __device__ __forceinline__ bool mg_tag_same(const MgTag& a, const MgTag& b) {
-  return a.magic == b.magic && a.minv == b.minv && a.omega == b.omega && a.levels == b.levels && a.level == b.level &&
-         a.nodes == b.nodes && a.real_bytes == b.real_bytes && a.pre_sweeps == b.pre_sweeps &&
-         a.post_sweeps == b.post_sweeps && a.coarse_sweeps == b.coarse_sweeps;
+  // no short circuits: the loads together
+  return (a.magic == b.magic) & (a.minv == b.minv) & (a.omega == b.omega) & (a.levels == b.levels) &
+         (a.level == b.level) & (a.nodes == b.nodes) & (a.real_bytes == b.real_bytes) & (a.pre_sweeps == b.pre_sweeps) &
+         (a.post_sweeps == b.post_sweeps) & (a.coarse_sweeps == b.coarse_sweeps);
+}
+
+// The first level that this solve applies as the dense operator (num_levels: none is there for it).
+template <typename R>
+__device__ __forceinline__ int mg_dense_from(const cpfem_mg_t& mg) {
+  const int lb = mg_dense_level(mg, sizeof(R));
+  if (lb >= mg.num_levels) return mg.num_levels;
+  return mg_tag_same(*mg_tag(mg), mg_tag_of<R>(mg, MgArrays<R>{mg, nullptr}.minv(lb), lb)) ? lb : mg.num_levels;
 }
 
 constexpr size_t kMgStageBytes = 220 * 1024;    // shared memory of a dense set-up's block, at most
@@ -476,8 +485,7 @@ __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg,
   // the coarse levels' nodes go to the warps of all blocks in turn, eight to a warp
   const int q = lane & 3;
   const int64_t tq = 8 * ((int64_t)wid * tm.nb + rank) + (lane >> 2), sq = 8 * (int64_t)warps * tm.nb;
-  int lb = mg_dense_level(mg, sizeof(R));
-  if (lb < L && !mg_tag_same(*mg_tag(mg), mg_tag_of<R>(mg, A.minv(lb), lb))) lb = L;
+  const int lb = sh.lb;
   auto barrier = [&]() { pt_reduce<0>(nullptr, 0, tm, a, sh); };
   const R* Mi0 = A.minv(0);
   // one sweep of level 0 after its row sums: f(node, X + om D^-1 (v - A X))

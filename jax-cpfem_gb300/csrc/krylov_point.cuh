@@ -28,7 +28,8 @@ struct PointArgs {
   double *phat, *shat;          // 3 * num_nodes each: what the neighbours gather
   double* cells;                // kPointCellBytes
   unsigned int* counters;       // kPointCounterBytes, zeroed before the launch
-  int* error;                   // zeroed before the launch
+  int* error;                   // set by a block that waited too long; zeroed before the launch (the report's
+                                // own word for a single system)
   const PointTeam* teams;       // by team_of_block, or null: one team of all blocks
   const int* team_of_block;
   cpfem_solve_report_t* out;    // single system: the launch's report
@@ -40,6 +41,7 @@ struct PointArgs {
   int smem_bytes;               // dynamic shared memory of a block
   double* vectors[8];           // multigrid: the Krylov vectors (3 * num_nodes each) where they do not
                                 // fit in shared memory, else null
+  int polls;                    // of a wait, at most
 };
 
 // How a solve is laid out: blocks, slot lanes per node; ok = false where the vectors do not

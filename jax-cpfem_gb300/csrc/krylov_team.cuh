@@ -18,7 +18,7 @@
 // 1 cell 30 -> 17, 10^3 57 -> 19, 16^3 60 -> 20, 24^3 60 -> 33, 32^3 61 -> 51, 40^3 116 -> 87.
 // Every sum has a fixed order, so a solve is bitwise reproducible, and all blocks of a team
 // hold the same scalars and take the same branch.  Polls are bounded: a block that waits too
-// long sets the error flag, stops, and the solve returns CPFEM_ERR_SOLVE.
+// long sets the error flag, on which all waits end, and the solve returns CPFEM_ERR_SOLVE.
 #pragma once
 
 #include <type_traits>
@@ -63,7 +63,6 @@ __global__ void k_precond_setup(const cpfem_sell_t L, const double* __restrict__
 struct PtTeam {
   int first, nb, id;
   unsigned int seq;   // barriers crossed
-  bool ok;
 };
 
 struct PtShared {
@@ -71,7 +70,8 @@ struct PtShared {
   double sum[kPointMaxValues];
   double alpha, omega, beta;
   double rho, rho_new, rs, atol2, cap;             // thread 0's
-  int bad, steps, k, go, early, restart;
+  int bad, steps, k, go, early, restart;           // bad: a wait of this block ran out
+  int lb;                                          // multigrid: mg_dense_from
 };
 
 // One warp adds v[0 .. n) in a fixed order; the result is valid in lane 0.
@@ -95,7 +95,9 @@ __device__ __forceinline__ double pt_warp_total(const double* v, int n) {
 // block order, so all hold the same bits.  The FP64 pipe is why: a warp instruction takes it
 // 64 cycles, and a shuffle tree in all 16 warps costs more of it than the vector work it sums.
 // The barrier is a counter that only grows (zeroed before the launch): one arrival per block,
-// one polling warp per value.
+// one polling warp per value.  Every 64th poll looks at the error word too, so once a block has
+// waited too long all other waits, and its own later ones in the iteration, end within
+// microseconds.  (Testing sh.bad here instead cost the multigrid kernel 2 to 5 %.)
 template <int NV>
 __device__ __forceinline__ void pt_reduce(const double* v, int active, PtTeam& tm, const PointArgs& a, PtShared& sh) {
   constexpr int NC = NV > 0 ? NV : 1;
@@ -126,9 +128,11 @@ __device__ __forceinline__ void pt_reduce(const double* v, int active, PtTeam& t
     if (lane == 0) {
       unsigned int c;
       int spins = 0;
-      do {
+      for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
-      } while (c < target && ++spins < kPtSpinLimit);
+        if (c >= target) break;
+        if ((++spins & 63) == 0 && (spins >= a.polls || *(volatile int*)a.error != 0)) break;
+      }
       if (c < target) {
         atomicExch(a.error, 1);
         sh.bad = 1;
@@ -150,7 +154,6 @@ __device__ __forceinline__ void pt_reduce(const double* v, int active, PtTeam& t
     }
   }
   __syncthreads();
-  if (sh.bad) tm.ok = false;
 }
 
 __device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
@@ -341,6 +344,8 @@ __device__ __noinline__ void pt_product_call(const PointArgs& a, const PtLocal B
 template <bool TRANS, int QL, typename R>
 __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg, const PtLocal& B, const double* v, double* hat,
                           double* out, R* y, PtTeam& tm, PtShared& sh);
+template <typename R>
+__device__ __forceinline__ int mg_dense_from(const cpfem_mg_t& mg);
 
 struct NoMg {};   // the preconditioner argument of the point kernel
 
@@ -354,7 +359,7 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
   extern __shared__ __align__(16) unsigned char pt_smem[];
   __shared__ PtShared sh;
   const int threads = (int)blockDim.x;
-  PtTeam tm{0, (int)gridDim.x, 0, 0u, true};
+  PtTeam tm{0, (int)gridDim.x, 0, 0u};
   int64_t t0 = 0, t1 = a.L.num_nodes;
   int job = 0;
   if (a.teams != nullptr) {
@@ -386,7 +391,11 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
       for (int i = 0; i < 8; ++i) *vs[i] = a.vectors[i] + 3 * B.n0;
     }
   }
-  if (threadIdx.x == 0) { sh.bad = 0; sh.steps = 0; }
+  if (threadIdx.x == 0) {
+    sh.bad = 0;
+    sh.steps = 0;
+    if constexpr (kMg) sh.lb = mg_dense_from<MR>(mg);
+  }
   __syncthreads();
   // slots per lane, and whether the block's rows fit beside the vectors
   for (int k = threadIdx.x; k < nn; k += threads)
@@ -513,7 +522,7 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
 
   double true_rs = -1.0;
   for (;;) {
-    while (tm.ok && sh.go) {
+    while (!sh.bad && sh.go) {
       {
         const double beta = sh.beta, omega = sh.omega;
         for (int d = threadIdx.x; d < nd; d += threads) p[d] = r[d] + beta * (p[d] - omega * q[d]);
@@ -587,14 +596,14 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
         }
       }
       __syncthreads();
-      if (sh.restart && tm.ok) {
+      if (sh.restart && !sh.bad) {
         for (int d = threadIdx.x; d < nd; d += threads) a.x[3 * B.n0 + d] = xs[d];
         pt_reduce<0>(nullptr, active, tm, a, sh);
         restart();
       }
     }
     for (int d = threadIdx.x; d < nd; d += threads) a.x[3 * B.n0 + d] = xs[d];
-    if (!(a.true_res || a.max_restarts > 0) || !tm.ok) break;
+    if (!(a.true_res || a.max_restarts > 0) || sh.bad) break;
     double vt[1] = {0.0};
     pt_reduce<0>(nullptr, active, tm, a, sh);
     product(a.x, t);
@@ -611,7 +620,7 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
       sh.restart = restarts < a.max_restarts && sh.k >= 0 && sh.k < a.maxiter && !pt_greater(sh.rs, sh.atol2) &&
                    pt_greater(true_rs, 100.0 * sh.atol2);
     __syncthreads();
-    if (!sh.restart || !tm.ok) break;
+    if (!sh.restart || sh.bad) break;
     restart();
   }
   if ((int)blockIdx.x == tm.first && threadIdx.x == 0) {
@@ -619,7 +628,6 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
       a.out->true_rs = a.true_res ? true_rs : -1.0;
       a.out->restarts = restarts;
       a.out->k = sh.k;
-      a.out->error = tm.ok ? 0 : 1;
       a.out->rs = sh.rs;
       a.out->atol2 = sh.atol2;
       a.out->rho = sh.rho;
