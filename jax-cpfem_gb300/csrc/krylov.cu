@@ -238,8 +238,9 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double* partials, G
 
 // The streaming kernel of the point preconditioners, for systems too large for the shared-memory
 // one (krylov_team.cuh): one thread per node, vectors in the workspace, blocks of four warps
-// per sub-partition that hide the row products' loads.
-template <bool TRANS>
+// per sub-partition that hide the row products' loads.  RESTARTS: max_restarts > 0; the code that
+// forms b - A x again costs the transposed product 2 % where it is only compiled in.
+template <bool TRANS, bool RESTARTS>
 __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L, const double* __restrict__ vals,
                                                            const double* __restrict__ b, double* __restrict__ x,
                                                            KWork w, int precond, double tol, double atol,
@@ -366,10 +367,10 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
     rho = rho_new;
     rho_new = vr[1];
     rs = vr[0];
-    if (kn < 0 && restarts < max_restarts && ok && rs > atol2) {
-      // restart at the current x: rhat = p = q = r = b - A x (x is complete: the last
-      // reduction crossed the grid barrier after every block wrote its part)
-      ++restarts;
+    // With restarts allowed: at a breakdown, and where the recursive residual met the stop rule but
+    // the true one is ten times above it, restart at the current x (rhat = p = q = r = b - A x; x is
+    // complete: the last reduction crossed the grid barrier after every block wrote its part).
+    if (RESTARTS && restarts < max_restarts && ok && (kn < 0 ? rs > atol2 : rs <= atol2 && kn < maxiter)) {
       double v3[1] = {0.0};
       for (int64_t a = t0; a < n; a += stride) {
         double acc[3];
@@ -383,9 +384,12 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
         }
       }
       ok = grid_reduce<1>(v3, parts(), w.sync, gen, smem, bcast) && ok;
-      rs = v3[0];
-      rho_new = v3[0];
-      rho = alpha = omega = 1.0;
+      if (kn < 0 || v3[0] > 100.0 * atol2) {
+        ++restarts;
+        rs = v3[0];
+        rho_new = v3[0];
+        rho = alpha = omega = 1.0;
+      }
       k = k + 1;
     } else {
       k = kn;
@@ -505,7 +509,7 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
     CPFEM_CUDA_TRY(cudaGetLastError());
   }
   int per_sm = 0, sms = 0;
-  const void* kfn = (const void*)k_bicgstab<TRANS>;
+  const void* kfn = max_restarts > 0 ? (const void*)k_bicgstab<TRANS, true> : (const void*)k_bicgstab<TRANS, false>;
   int rc = sm_count_and_blocks(kfn, &per_sm, &sms);
   if (rc) return rc;
   if (per_sm < 1) {

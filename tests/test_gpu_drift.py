@@ -1,0 +1,33 @@
+"""Restarts of a solve whose recursive residual has drifted below its true one, in the
+shared-memory kernel (all SMs) and in the streaming one (a single block: 12^3 cells' vectors do not
+fit its shared memory)."""
+import numpy as np
+import pytest
+import torch
+
+from tests.test_gpu_point_solver import _residual, _system
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(solver_mod, prob, A, b, precond, grid_blocks, tol, restarts):
+    """(relative true residual, iterations, restarts made)"""
+    x, k, ok = solver_mod.bicgstab(prob, A, b, torch.zeros_like(b), precond=precond, tol=tol, atol=1e-300,
+                                   restarts=restarts, grid_blocks=grid_blocks, maxiter=4000)
+    st = np.zeros(9)
+    assert ok and prob.lib.cpfem_bicgstab_last_stats_ex(st.ctypes.data, 9) == 0
+    return _residual(A, x, b) / float(b.norm()), k, int(st[6])
+
+
+@pytest.mark.parametrize("grid_blocks", [0, 1])
+@pytest.mark.parametrize("precond", [1, 2])
+def test_drifted_solve_restarts(pkg, gpu, grid_blocks, precond):
+    """At 1e-13 the recursion claims convergence with the true residual 20 times above the limit; a
+    restart brings it within the rule's factor of 10."""
+    problem_mod, solver_mod = gpu
+    prob, A, _, _ = _system(pkg, problem_mod, solver_mod, (12, 12, 12))
+    b = torch.sin(3.0 + torch.arange(3 * prob.num_nodes, dtype=torch.float64, device="cuda"))
+    plain, _, none = _solve(solver_mod, prob, A, b, precond, grid_blocks, 1e-13, 0)
+    assert none == 0 and plain > 1e-12
+    rn, _, made = _solve(solver_mod, prob, A, b, precond, grid_blocks, 1e-13, 20)
+    assert 1 <= made <= 3 and rn <= 1e-12
