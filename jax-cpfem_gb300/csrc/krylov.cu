@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
   const double atol2 = fmax(tol * tol * v2[0], atol * atol);
   if (blockIdx.x == 0 && threadIdx.x == 0) w.out->bb = v2[0];   // b.b, written now: nothing stays live
   double rs = v2[1], rho_new = v2[1], rho = 1.0, alpha = 1.0, omega = 1.0;
+  double drift = INFINITY;
   int k = 0, restarts = 0;
 
   while (ok && rs > atol2 && k < maxiter && k >= 0) {
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
     rho_new = vr[1];
     rs = vr[0];
     // With restarts allowed: at a breakdown, and where the recursive residual met the stop rule but
-    // the true one is ten times above it, restart at the current x (rhat = p = q = r = b - A x; x is
+    // the true one is ten times above it and half what it was there last, restart at the current x (rhat = p = q = r = b - A x; x is
     // complete: the last reduction crossed the grid barrier after every block wrote its part).
     if (RESTARTS && restarts < max_restarts && ok && (kn < 0 ? rs > atol2 : rs <= atol2 && kn < maxiter)) {
       double v3[1] = {0.0};
@@ -384,7 +385,8 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
         }
       }
       ok = grid_reduce<1>(v3, parts(), w.sync, gen, smem, bcast) && ok;
-      if (kn < 0 || v3[0] > 100.0 * atol2) {
+      if (kn < 0 || (v3[0] > 100.0 * atol2 && 4.0 * v3[0] < drift)) {
+        if (kn >= 0) drift = v3[0];
         ++restarts;
         rs = v3[0];
         rho_new = v3[0];

@@ -69,7 +69,7 @@ struct PtShared {
   double part[kPointMaxValues][kPtMaxThreads];     // the threads' partial sums
   double sum[kPointMaxValues];
   double alpha, omega, beta;
-  double rho, rho_new, rs, atol2, cap;             // thread 0's
+  double rho, rho_new, rs, atol2, cap, drift;      // thread 0's
   int bad, steps, k, go, early, restart;           // bad: a wait of this block ran out
   int lb;                                          // multigrid: mg_dense_from
 };
@@ -505,6 +505,7 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
     sh.k = 0;
     sh.go = pt_greater(sh.rs, sh.atol2) && a.maxiter > 0;
     sh.cap = 1e16 * fmax(sh.rs, sh.atol2);
+    sh.drift = __longlong_as_double(0x7FF0000000000000ll);
   }
   __syncthreads();
 
@@ -615,10 +616,14 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
     true_rs = sh.sum[0];
     // Where restarts are allowed, a recursive residual that met the stop rule while the true one
     // is ten times above it (a near-singular system drives it through values so large that it
-    // drifts from b - A x) is a breakdown too.
-    if (threadIdx.x == 0)
+    // drifts from b - A x) is a breakdown too, as long as each such restart halves the true one:
+    // below FP64's reach of the system they would go on to max_restarts for nothing (12^3 cells at
+    // 1e-14: 428 iterations, 184 without).
+    if (threadIdx.x == 0) {
       sh.restart = restarts < a.max_restarts && sh.k >= 0 && sh.k < a.maxiter && !pt_greater(sh.rs, sh.atol2) &&
-                   pt_greater(true_rs, 100.0 * sh.atol2);
+                   pt_greater(true_rs, 100.0 * sh.atol2) && pt_greater(sh.drift, 4.0 * true_rs);
+      sh.drift = true_rs;
+    }
     __syncthreads();
     if (!sh.restart || sh.bad) break;
     restart();

@@ -31,3 +31,16 @@ def test_drifted_solve_restarts(pkg, gpu, grid_blocks, precond):
     assert none == 0 and plain > 1e-12
     rn, _, made = _solve(solver_mod, prob, A, b, precond, grid_blocks, 1e-13, 20)
     assert 1 <= made <= 3 and rn <= 1e-12
+
+
+@pytest.mark.parametrize("grid_blocks", [0, 1])
+@pytest.mark.parametrize("precond", [1, 2])
+def test_unattainable_tolerance_ends_the_restarts(pkg, gpu, grid_blocks, precond):
+    """1e-15 is below what FP64 reaches on this system: the restarts end when one no longer halves
+    the true residual, which starts 2e-12 and stops near 1e-12."""
+    problem_mod, solver_mod = gpu
+    prob, A, _, _ = _system(pkg, problem_mod, solver_mod, (12, 12, 12))
+    b = torch.sin(3.0 + torch.arange(3 * prob.num_nodes, dtype=torch.float64, device="cuda"))
+    plain, k0, _ = _solve(solver_mod, prob, A, b, precond, grid_blocks, 1e-15, 0)
+    rn, k, made = _solve(solver_mod, prob, A, b, precond, grid_blocks, 1e-15, 20)
+    assert rn <= plain and 1 <= made <= 4 and k < 2 * k0
