@@ -106,13 +106,16 @@ typedef struct {
                                    s_warm + ds/dF : (F - s_f) instead of at s_warm;
                                  2: Newton directions from an FP32 Jacobian / LU while the
                                    Jacobian's scale max_a d(dgamma_a)/d(tau_a) C11 <= 1e4
-                                   (else FP64), and, with s_warm, the start itself improved
-                                   by Newton steps in FP32 alone; the residual, its stop test and the tangent
+                                   (else FP64); the residual, its stop test and the tangent
                                    stay FP64, so the converged state is the same root;
                                  4: the consistent tangent (dP/dF, and ds/dF for the
                                    prediction) in FP32 under the same scale test (else
                                    FP64): it is only the global Newton's Jacobian, so the
-                                   converged solution is unchanged.
+                                   converged solution is unchanged;
+                                 8 (with s_warm): the start is first moved to the root by
+                                   Newton steps in FP32 alone, as far as FP32 resolves it; the
+                                   FP64 iteration then starts there and ends at the root of its
+                                   own residual to its own tolerance.
                                  0 with s_warm = NULL: the reference's iterates. */
   const int32_t* order;       /* [num_gp] permutation or NULL (no cell list): thread t
                                  evaluates GP order[t].  Ordering GPs by their previous

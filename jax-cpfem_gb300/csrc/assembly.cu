@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kGpThreads) k_gp_eval(const __grid_constant__ 
     }
   }
   cp_local_newton<NS, kGpThreads>(m, cc, Ct, m.ao * a.dt, 1.0 / xm, st, a.s_warm != nullptr ? s0 : nullptr,
-                                  (a.local_flags & 2) != 0);
+                                  (a.local_flags & 2) != 0, (a.local_flags & 8) != 0);
   if (a.s_warm != nullptr) {
     if (st.rn <= m.local_tol) {
 #pragma unroll

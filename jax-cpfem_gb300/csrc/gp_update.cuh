@@ -409,7 +409,7 @@ constexpr int kWarmStartIters = 8;   // a warm start still unconverged after thi
 // residuals at s + relax ds, relax = 1, 1/2, ..., until the norm drops below the current
 // one or max_sub_step trials were made; the last trial is taken.  It starts from s0 = 0,
 // as the reference does, or -- given s_init, the same GP's last converged stress -- from
-// there, which needs far fewer iterations once the global Newton iterates settle; with j32 the
+// there, which needs far fewer iterations once the global Newton iterates settle; with pre32 the
 // FP32 pre-solve above moves that start to the root first, as far as FP32 resolves it.  A
 // warm start that has not converged after kWarmStartIters iterations (or went
 // non-finite) is abandoned: one step with a single trial evaluates the residual at
@@ -418,7 +418,8 @@ constexpr int kWarmStartIters = 8;   // a warm start still unconverged after thi
 // step, the restart and the pre-solve's included.  1/g is in the slab.
 template <int NS, int TH>
 __device__ __forceinline__ void cp_local_newton(const MatDev& m, const Cub& cc, const double* Ct, double cdt, double pexp,
-                                                GPSolve& st, const double* s_init = nullptr, bool j32 = false) {
+                                                GPSolve& st, const double* s_init = nullptr, bool j32 = false,
+                                                bool pre32 = false) {
   const int ie1 = int_exponent(pexp - 1.0);
   double r[6], st_s[6], ds[6];
   bool warm = s_init != nullptr;
@@ -428,7 +429,7 @@ __device__ __forceinline__ void cp_local_newton(const MatDev& m, const Cub& cc, 
     ds[k] = 0.0;
   }
   int pre = 0;
-  if (warm && j32) {
+  if (warm && pre32) {
     PreIn in;
     constexpr int I6[6] = {0, 4, 8, 5, 2, 1};
     bool fits = true;       // NaN or beyond FP32: left to the FP64 iteration

@@ -230,6 +230,8 @@ class CrystalPlasticity:
         # Newton directions of the local solve from an FP32 Jacobian while its scale allows
         # (same residual, stop test and tangent in FP64: same converged state)
         self.fp32_local_jacobian = True
+        # ... and, beside them, first moves a warm start to the root by Newton steps in FP32 alone
+        self.fp32_local_presolve = True
         # the consistent tangent (the global Newton's Jacobian) in FP32 where the local
         # Jacobian's scale allows; the residual and the converged state stay FP64
         self.fp32_tangent = False
@@ -621,7 +623,7 @@ class CrystalPlasticity:
                  **outs):
         """cpfem_gp_args_t of one constitutive pass.  predict: start the local Newton at the
         linear prediction (needs the warm-start arrays); fast_local: FP32 Newton directions
-        (the problem's ``fp32_local_jacobian`` decides)."""
+        and pre-solve (the problem's ``fp32_local_jacobian`` and ``fp32_local_presolve`` decide)."""
         a = _capi.GPArgs()
         fpi, g, slip, rot_table, rot_idx, param_table, param_idx = state
         a.num_gp = self.num_gp if num_gp is None else num_gp
@@ -641,7 +643,8 @@ class CrystalPlasticity:
             a.elastic_table = _dev_ptr(self.elastic_table) if param_table is self.param_table else None
         a.weight_jxw = 1 if outs.pop("weight_jxw", False) else 0
         a.local_flags = (1 if predict else 0) | (2 if (fast_local and self.fp32_local_jacobian) else 0) | \
-            (4 if (fast_local and self.fp32_tangent) else 0)
+            (4 if (fast_local and self.fp32_tangent) else 0) | \
+            (8 if (fast_local and self.fp32_local_jacobian and self.fp32_local_presolve) else 0)
         cl = outs.pop("cell_list", None)
         if cl is not None:
             a.cell_list, a.num_listed = _dev_ptr(cl), int(cl.numel())
