@@ -342,11 +342,11 @@ __device__ __forceinline__ float cp_residual_f32(const MatDev& m, const PreIn& i
                2.0f * fmaf(r[3], r[3], fmaf(r[4], r[4], r[5] * r[5])));
 }
 
-// Damped Newton: a step is halved until the residual is finite and smaller.  Returns the start
-// itself where that is near the root already, or where it or the equation is not finite in FP32;
-// steps counts the steps taken.
+// Damped Newton, `most` steps (at least 1) and kPreIters at most: a step is halved until the
+// residual is finite and smaller.  Returns the start itself where that is near the root already, or
+// where it or the equation is not finite in FP32; steps counts the steps taken.
 template <int NS, int TH>
-__device__ __noinline__ Vec6<float> cp_presolve(const MatDev& m, PreIn in, int* steps) {
+__device__ __noinline__ Vec6<float> cp_presolve(const MatDev& m, PreIn in, int most, int* steps) {
   Vec6<float> out;
   float s[6], st[6], ds[6], r[6], M[9];
   float rn = 0.0f, relax = 0.0f, size = 1.0f;
@@ -370,7 +370,7 @@ __device__ __noinline__ Vec6<float> cp_presolve(const MatDev& m, PreIn in, int* 
         s[k] = st[k];
         size = fmaxf(size, fabsf(s[k]));
       }
-      last = !(rt > kPreNear * size) || it + 1 >= kPreIters ||
+      last = !(rt > kPreNear * size) || it + 1 >= min(kPreIters, most) ||
              (rt > 0.3f * rn && rt < kPreFar * size);          // FP32's rounding has been reached
     } else {
       if (++trial >= kPreTrials) break;
@@ -415,7 +415,8 @@ constexpr int kWarmStartIters = 8;   // a warm start still unconverged after thi
 // non-finite) is abandoned: one step with a single trial evaluates the residual at
 // s0 = 0 and the reference's iteration runs from there with its own max_iter.  Either way
 // the result is the root of the same residual to the same tolerance.  st.iters counts every
-// step, the restart and the pre-solve's included.  1/g is in the slab.
+// step, the restart and the pre-solve's included: max_iter from each start at most.  1/g is in
+// the slab.
 template <int NS, int TH>
 __device__ __forceinline__ void cp_local_newton(const MatDev& m, const Cub& cc, const double* Ct, double cdt, double pexp,
                                                 GPSolve& st, const double* s_init = nullptr, bool j32 = false,
@@ -441,16 +442,17 @@ __device__ __forceinline__ void cp_local_newton(const MatDev& m, const Cub& cc, 
     }
     in.cdt = f32_of(cdt); in.pexp = f32_of(pexp); in.ie1 = ie1;
     in.cc = cub_of<float>(cc);
-    if (fits) {
-      const Vec6<float> p = cp_presolve<NS, TH>(m, in, &pre);
-      if (pre > 0)
+    // the pre-solve's steps count toward max_iter, one of which is left for the restart from 0
+    if (fits && m.max_iter > 1) {
+      const Vec6<float> p = cp_presolve<NS, TH>(m, in, m.max_iter - 1, &pre);
 #pragma unroll
-        for (int k = 0; k < 6; ++k) st_s[k] = f64_of(p.v[k]);
+      for (int k = 0; k < 6; ++k)
+        if (p.v[k] != in.s[k]) st_s[k] = f64_of(p.v[k]);      // an unmoved start keeps its FP64 digits
     }
   }
-  const int warm_iters = (kWarmStartIters < m.max_iter) ? kWarmStartIters : m.max_iter - 1;
+  const int warm_iters = min(kWarmStartIters, m.max_iter - 1 - pre);
   // one residual evaluation per pass of the loop: the start's (it = -1), or a trial's of step it
-  int it = -1, it0 = 0;   // it0: the step the s0 = 0 iteration started at
+  int it = -1, it0 = -pre;   // it0: the step the s0 = 0 iteration started at
   int sub = 0, sub_cap = 1;
   double relax = 1.0, rn0 = 0.0;
   for (;;) {

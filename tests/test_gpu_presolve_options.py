@@ -46,3 +46,26 @@ def test_pre_solve_can_be_left_out(pkg, gpu, spec_name):
     assert float((r1 - r0).abs().max() / r0.abs().max()) < 1e-9
     assert float((v1 - v0).abs().max() / v0.abs().max()) < 1e-9
     assert torch.equal(out[False, True][0], out[False, False][0]) and torch.equal(out[False, True][2], out[False, False][2])
+
+
+@pytest.mark.parametrize("max_iter", [1, 2, 3, 6, 300])
+@pytest.mark.parametrize("spec_name", ["BENCH_STEEL", "BENCH_TANTALUM"])
+def test_pre_solve_steps_count_toward_max_iter(pkg, gpu, spec_name, max_iter):
+    """From a far start: max_iter steps of any kind from the warm start, the step back to S = 0 among
+    them, and max_iter more from there; what fails then fails, and what the pass from S = 0 reaches
+    in max_iter steps is reached."""
+    problem_mod, _ = gpu
+    spec = getattr(pkg.material, spec_name)
+    prob, u, root = _problem(pkg, problem_mod, spec)
+    prob.mat_c.max_iter = max_iter
+    prob.warm_start_local = False
+    res, _, status = prob.assemble(u)
+    cold, cold_status = res.clone(), int(status.item())
+    prob.warm_start_local = True
+    for start in (3.0 * root, -root, 1e30 * root):
+        r, _, its, status = _run(prob, u, start)
+        assert int(its.max()) <= 2 * max_iter
+        if cold_status == 0:
+            assert status == 0 and float((r - cold).abs().max() / cold.abs().max()) < 1e-9
+        if max_iter == 1:                 # no pre-solve, the step back to S = 0, one step
+            assert torch.equal(r, cold) and status == cold_status
