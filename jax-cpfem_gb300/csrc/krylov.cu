@@ -6,7 +6,7 @@
 // the SpMV's limit, and a shuffle reduction would cost as many FP64 adds as the FMAs.
 //
 // BiCGSTAB runs as one cooperative launch.  Systems whose vectors fit the blocks' shared
-// memory, and every multigrid solve, use the kernel of krylov_team.cuh; the kernels here
+// memory use the kernel of krylov_team.cuh; the kernels here
 // stream their vectors from memory, for larger systems and for batches of many.  In them
 // every block owns a fixed set of nodes, the five global dependencies of an iteration (the halo of phat and shat, four dot
 // products) are crossed with a grid barrier, and every block reduces the per-block
@@ -21,7 +21,7 @@
 #include <string>
 
 #include "cpfem_common.cuh"
-#include "krylov_team.cuh"
+#include "krylov_mg.cuh"
 #include "reduce.cuh"
 
 namespace cpfem {
@@ -236,15 +236,89 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double* partials, G
   return ok;
 }
 
-// The streaming kernel of the point preconditioners, for systems too large for the shared-memory
-// one (krylov_team.cuh): one thread per node, vectors in the workspace, blocks of four warps
-// per sub-partition that hide the row products' loads.  RESTARTS: max_restarts > 0; the code that
-// forms b - A x again costs the transposed product 2 % where it is only compiled in.
-template <bool TRANS, bool RESTARTS>
-__global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L, const double* __restrict__ vals,
-                                                           const double* __restrict__ b, double* __restrict__ x,
-                                                           KWork w, int precond, double tol, double atol,
-                                                           int maxiter, int max_restarts) {
+// One V-cycle out = M^-1 in of the streaming kernel, in precision R, level 0 a thread per node: node
+// a is thread a's of the grid, as in the rest of the kernel, so `in` and `out` need no barrier of
+// their own.  b: room for 3 kMgDenseNodes values in shared memory.
+template <bool TRANS, typename R>
+__device__ __forceinline__ void mg_vcycle_streaming(const cpfem_mg_t& mg, const double* vals, const double* in, double* out,
+                                                    R* b, int lb, GridSync* gs, unsigned int& gen, bool& ok) {
+  const MgArrays<R> A{mg, vals};
+  const cpfem_sell_t& S = mg.sell[0];
+  const R* Mi = A.minv(0);
+  const R om = (R)mg.omega;
+  const int64_t n = S.num_nodes, stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  auto barrier = [&]() { ok = grid_barrier(gs, gen) && ok; };
+  // X + om D^-1 (in - A X) at node a
+  auto sweep = [&](const R* X, int64_t a, R* z) {
+    R acc[3], r[3];
+    sell_rows<TRANS, true, R, double>(S, vals, X, a, acc);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) r[i] = to_prec<R>(in[3 * a + i]) - acc[i];
+    mg_apply_minv<TRANS>(Mi, a, r, z);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) z[i] = mad(om, z[i], __ldcg(&X[3 * a + i]));
+  };
+  R *X = A.x(0), *T = A.t(0);
+  for (int64_t a = t0; a < n; a += stride) {
+    R v[3], z[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[i] = to_prec<R>(in[3 * a + i]);
+    mg_apply_minv<TRANS>(Mi, a, v, z);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) X[3 * a + i] = om * z[i];
+  }
+  for (int k = 1; k < mg.pre_sweeps; ++k) {
+    barrier();
+    for (int64_t a = t0; a < n; a += stride) {
+      R z[3];
+      sweep(X, a, z);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) T[3 * a + i] = z[i];
+    }
+    R* tmp = X; X = T; T = tmp;
+  }
+  barrier();
+  R* Res = A.r(0);
+  for (int64_t a = t0; a < n; a += stride) {
+    R acc[3];
+    sell_rows<TRANS, true, R, double>(S, vals, X, a, acc);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const R rv = to_prec<R>(in[3 * a + i]) - acc[i];
+      Res[3 * a + i] = (mg.free_dof != nullptr && mg.free_dof[3 * a + i] == 0) ? R(0) : rv;
+    }
+  }
+  barrier();
+  const R* X1 = mg_coarse_levels<TRANS, R>(mg, A, lb, t0 >> 2, stride >> 2, (int)(t0 & 3), blockIdx.x, gridDim.x, b, barrier);
+  barrier();
+  mg_prolong(mg, 0, X, X1, t0, stride, n);
+  for (int k = 0; k < mg.post_sweeps; ++k) {
+    barrier();
+    for (int64_t a = t0; a < n; a += stride) {
+      R z[3];
+      sweep(X, a, z);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) T[3 * a + i] = z[i];
+    }
+    R* tmp = X; X = T; T = tmp;
+  }
+  for (int64_t a = t0; a < n; a += stride)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) out[3 * a + i] = to_f64(X[3 * a + i]);
+}
+
+// The streaming kernel, for systems too large for the shared-memory one (krylov_team.cuh): one
+// thread per node, vectors in the workspace.  Three blocks a SM, six warps per sub-partition, hide
+// the row products' loads; with the FP32 V-cycle one block of the whole register file does that
+// better.  RESTARTS: max_restarts > 0; the code that forms b - A x again costs the transposed product
+// 2 % where it is only compiled in.  MR: void for a point preconditioner (precond), or the
+// V-cycle's precision.
+template <bool TRANS, bool RESTARTS, typename MR, typename MG>
+__global__ void __launch_bounds__(kPThreads, std::is_same<MR, float>::value ? 1 : 3) k_bicgstab(
+    const cpfem_sell_t L, const double* __restrict__ vals, const double* __restrict__ b, double* __restrict__ x,
+    KWork w, int precond, double tol, double atol, int maxiter, int max_restarts, const __grid_constant__ MG mg) {
+  constexpr bool kMg = !std::is_void<MR>::value;
   __shared__ double smem[4 * 32];
   __shared__ double bcast[4];
   const int64_t n = L.num_nodes;
@@ -258,6 +332,19 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
     return p;
   };
   bool ok = true;
+  __shared__ double drift;     // ||b - A x||^2 where the last drift was seen
+  if (threadIdx.x == 0) drift = INFINITY;
+  // out = M v at this thread's nodes, by the V-cycle
+  __shared__ double dense_b[kMg ? 3 * kMgDenseNodes : 1];
+  __shared__ int lb;
+  if constexpr (kMg) {
+    if (threadIdx.x == 0) lb = mg_dense_from<MR>(mg);
+    __syncthreads();
+  }
+  auto vcycle = [&](const double* v, double* out) {
+    if constexpr (kMg)
+      mg_vcycle_streaming<TRANS, MR>(mg, vals, v, out, reinterpret_cast<MR*>(dense_b), lb, w.sync, gen, ok);
+  };
 
   // r = b - A x0 ; rhat = p = q = r
   double v2[2] = {0.0, 0.0};
@@ -277,8 +364,9 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
   ok = grid_reduce<2>(v2, parts(), w.sync, gen, smem, bcast) && ok;
   const double atol2 = fmax(tol * tol * v2[0], atol * atol);
   if (blockIdx.x == 0 && threadIdx.x == 0) w.out->bb = v2[0];   // b.b, written now: nothing stays live
+  double cap = 0.0;
+  if constexpr (std::is_same<MR, float>::value) cap = 1e16 * fmax(v2[1], atol2);
   double rs = v2[1], rho_new = v2[1], rho = 1.0, alpha = 1.0, omega = 1.0;
-  double drift = INFINITY;
   int k = 0, restarts = 0;
 
   while (ok && rs > atol2 && k < maxiter && k >= 0) {
@@ -292,10 +380,13 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
         pv[i] = w.r[d] + beta * (w.p[d] - omega * w.q[d]);
         w.p[d] = pv[i];
       }
-      apply_m(precond, w.minv, a, pv, ph);
+      if constexpr (!kMg) {
+        apply_m(precond, w.minv, a, pv, ph);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) w.phat[3 * a + i] = ph[i];
+        for (int i = 0; i < 3; ++i) w.phat[3 * a + i] = ph[i];
+      }
     }
+    vcycle(w.p, w.phat);
     ok = grid_barrier(w.sync, gen) && ok;
     // q = A phat ; alpha = rho_new / (rhat . q)
     double v1[1] = {0.0};
@@ -322,10 +413,13 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
         w.s[d] = sv[i];
         vs[0] = fma(sv[i], sv[i], vs[0]);
       }
-      apply_m(precond, w.minv, a, sv, sh);
+      if constexpr (!kMg) {
+        apply_m(precond, w.minv, a, sv, sh);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) w.shat[3 * a + i] = sh[i];
+        for (int i = 0; i < 3; ++i) w.shat[3 * a + i] = sh[i];
+      }
     }
+    vcycle(w.s, w.shat);
     ok = grid_reduce<1>(vs, parts(), w.sync, gen, smem, bcast) && ok;   // also the shat halo barrier
     // t = A shat ; omega = (t.s)/(t.t)
     double vt[2] = {0.0, 0.0};
@@ -368,10 +462,11 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
     rho = rho_new;
     rho_new = vr[1];
     rs = vr[0];
+    if (std::is_same<MR, float>::value && !(rs <= cap)) kn = -12;      // as in k_bicgstab_team
     // With restarts allowed: at a breakdown, and where the recursive residual met the stop rule but
     // the true one is ten times above it and half what it was there last, restart at the current x (rhat = p = q = r = b - A x; x is
     // complete: the last reduction crossed the grid barrier after every block wrote its part).
-    if (RESTARTS && restarts < max_restarts && ok && (kn < 0 ? rs > atol2 : rs <= atol2 && kn < maxiter)) {
+    if (RESTARTS && restarts < max_restarts && ok && (kn < 0 ? kn != -12 && rs > atol2 : rs <= atol2 && kn < maxiter)) {
       double v3[1] = {0.0};
       for (int64_t a = t0; a < n; a += stride) {
         double acc[3];
@@ -385,8 +480,10 @@ __global__ void __launch_bounds__(kPThreads, 3) k_bicgstab(const cpfem_sell_t L,
         }
       }
       ok = grid_reduce<1>(v3, parts(), w.sync, gen, smem, bcast) && ok;
-      if (kn < 0 || (v3[0] > 100.0 * atol2 && 4.0 * v3[0] < drift)) {
-        if (kn >= 0) drift = v3[0];
+      const bool again = kn < 0 || (v3[0] > 100.0 * atol2 && 4.0 * v3[0] < drift);
+      __syncthreads();
+      if (kn >= 0 && threadIdx.x == 0) drift = v3[0];
+      if (again) {
         ++restarts;
         rs = v3[0];
         rho_new = v3[0];
@@ -475,8 +572,8 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
   KWork w;
   carve(workspace, L.num_nodes, &w);
   PointPlan plan{};
-  if (const int rc = point_plan(L.num_nodes, precond, TRANS, grid_blocks, &plan); rc != CPFEM_OK) return rc;
-  if (plan.ok || precond == 3) {
+  if (const int rc = point_plan(L.num_nodes, precond, precond == 3 && mgp->precision == 1, TRANS, grid_blocks, &plan); rc != CPFEM_OK) return rc;
+  if (plan.ok) {
     PointArgs a{};
     a.L = L; a.vals = vals; a.b = b; a.x = x;
     a.phat = w.phat; a.shat = w.shat;
@@ -493,10 +590,6 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
     CPFEM_CUDA_TRY(cudaMemsetAsync(w.sync, 0, (size_t)((char*)w.partials - (char*)w.sync) + 128, s));
     // the failure test: one arrival short (the count's first increment wraps it to 0)
     if (lost_polls > 0) CPFEM_CUDA_TRY(cudaMemsetAsync(a.counters, 0xFF, sizeof(unsigned int), s));
-    if (!plan.ok) {
-      double* const v[8] = {w.r, w.rhat, w.p, w.q, w.t, w.s, w.minv, w.minv + 3 * (size_t)L.num_nodes};
-      std::copy(v, v + 8, a.vectors);
-    }
     const int rc = precond == 3 ? mg_launch(plan, TRANS, a, *mgp, s) : point_launch(plan, TRANS, a, s);
     if (rc != CPFEM_OK) return rc;
     return finish_solve(w.out, info, flags, report, s);
@@ -511,7 +604,10 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
     CPFEM_CUDA_TRY(cudaGetLastError());
   }
   int per_sm = 0, sms = 0;
-  const void* kfn = max_restarts > 0 ? (const void*)k_bicgstab<TRANS, true> : (const void*)k_bicgstab<TRANS, false>;
+  const void* kfn = precond != 3 ? (max_restarts > 0 ? (const void*)k_bicgstab<TRANS, true, void, NoMg>
+                                                     : (const void*)k_bicgstab<TRANS, false, void, NoMg>)
+                    : mgp->precision == 1 ? (const void*)k_bicgstab<TRANS, true, float, cpfem_mg_t>
+                                          : (const void*)k_bicgstab<TRANS, true, double, cpfem_mg_t>;
   int rc = sm_count_and_blocks(kfn, &per_sm, &sms);
   if (rc) return rc;
   if (per_sm < 1) {
@@ -527,7 +623,9 @@ static int run_bicgstab(const cpfem_sell_t& L, const double* vals, const double*
   int pc = precond;
   double tl = tol, at = atol;
   int mi = maxiter, mr = max_restarts;
-  void* args[] = {&Lc, &vals, &bb, &xx, &w, &pc, &tl, &at, &mi, &mr};
+  cpfem_mg_t mg{};
+  if (precond == 3) mg = *mgp;
+  void* args[] = {&Lc, &vals, &bb, &xx, &w, &pc, &tl, &at, &mi, &mr, &mg};
   CPFEM_CUDA_TRY(cudaLaunchCooperativeKernel(kfn, dim3((unsigned)blocks), dim3(kPThreads), args, 0, s));
   if (flags & kKrylovTrueResidual) {
     // ||b - A x||^2 of the returned x: block partials, then one block sums them in order

@@ -471,13 +471,78 @@ __device__ R* mg_local_cycle(const cpfem_mg_t& mg, const MgArrays<R>& A, const M
   return at[lb];
 }
 
+// Levels 1 .. L-1 of a V-cycle.  Level 0's residual is complete in A.r(0); the iterate of level 1
+// that is returned is complete after the caller's next barrier.  tq, sq, q as in mgq_apply; rank of
+// nb blocks; b: room for 3 kMgDenseNodes values in shared memory.
+template <bool TRANS, typename R, class Barrier>
+__device__ __forceinline__ const R* mg_coarse_levels(const cpfem_mg_t& mg, const MgArrays<R>& A, int lb, int64_t tq,
+                                                     int64_t sq, int q, int rank, int nb, R* b, Barrier barrier) {
+  const int L = mg.num_levels;
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)blockDim.x >> 5;
+  R* at[CPFEM_MG_MAX_LEVELS];
+  // ---- levels 1 .. lb-1, down
+  for (int l = 1; l < lb; ++l) {
+    const R* V = A.values(l);
+    const R* Mi = A.minv(l);
+    R *X = A.x(l), *T = A.t(l);
+    mgq_restrict(mg, l - 1, (const R*)A.r(l - 1), A.b(l), tq, sq, q);
+    mgq_first_sweep<TRANS>(mg, Mi, l, X, (const R*)A.b(l), tq, sq, q);
+    const int nsw = (l == L - 1) ? mg.coarse_sweeps : mg.pre_sweeps;
+    for (int k = 1; k < nsw; ++k) {
+      barrier();
+      mgq_apply<TRANS>(mg, V, Mi, l, (const R*)X, T, (const R*)A.b(l), false, tq, sq, q);
+      R* tmp = X; X = T; T = tmp;
+    }
+    at[l] = X;
+    if (l == L - 1) break;
+    barrier();
+    mgq_apply<TRANS>(mg, V, Mi, l, (const R*)X, A.r(l), (const R*)A.b(l), true, tq, sq, q);
+    barrier();
+  }
+  // ---- levels lb .. L-1: the dense operator.  Every block restricts the whole right-hand side
+  // (a few KB of residual, L1's work) rather than wait for its parts; a warp per row.
+  if (lb < L) {
+    mgq_restrict(mg, lb - 1, (const R*)A.r(lb - 1), b, threadIdx.x >> 2, blockDim.x >> 2, q);
+    __syncthreads();
+    const int N = 3 * (int)mg.sell[lb].num_nodes;
+    const R* K = mg_dense<R>(mg);
+    R* X = A.x(lb);
+    const int r1 = (int)((int64_t)N * (rank + 1) / nb);
+    for (int row = (int)((int64_t)N * rank / nb) + wid; row < r1; row += warps) {
+      R acc = R(0);
+#pragma unroll 4
+      for (int c = lane; c < N; c += 32)
+        acc = mad(TRANS ? __ldg(&K[(size_t)c * N + row]) : __ldg(&K[(size_t)row * N + c]), b[c], acc);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) X[row] = acc;
+    }
+    at[lb] = X;
+  }
+  // ---- levels below the coarsest, up
+  for (int l = (lb < L ? lb : L - 1) - 1; l >= 1; --l) {
+    const R* V = A.values(l);
+    const R* Mi = A.minv(l);
+    R* X = at[l];
+    R* T = (X == A.x(l)) ? A.t(l) : A.x(l);
+    barrier();
+    if (q == 0) mg_prolong(mg, l, X, (const R*)at[l + 1], tq, sq, mg.sell[l].num_nodes);
+    for (int k = 0; k < mg.post_sweeps; ++k) {
+      barrier();
+      mgq_apply<TRANS>(mg, V, Mi, l, (const R*)X, T, (const R*)A.b(l), false, tq, sq, q);
+      R* tmp = X; X = T; T = tmp;
+    }
+    at[l] = X;
+  }
+  return at[1];
+}
+
 // One V-cycle hat = out = M^-1 v: v and hat are the block's dofs of FP64 vectors, out the global
 // vector that neighbours gather, y room for the block's row sums.
 template <bool TRANS, int QL, typename R>
 __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg, const PtLocal& B, const double* v, double* hat,
                           double* out, R* y, PtTeam& tm, PtShared& sh) {
   const MgArrays<R> A{mg, a.vals};
-  const int L = mg.num_levels;
   const R om = (R)mg.omega;
   const int threads = (int)blockDim.x, wid = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = threads >> 5;
   const int rank = (int)blockIdx.x - tm.first, nn = B.nn;
@@ -485,7 +550,6 @@ __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg,
   // the coarse levels' nodes go to the warps of all blocks in turn, eight to a warp
   const int q = lane & 3;
   const int64_t tq = 8 * ((int64_t)wid * tm.nb + rank) + (lane >> 2), sq = 8 * (int64_t)warps * tm.nb;
-  const int lb = sh.lb;
   auto barrier = [&]() { pt_reduce<0>(nullptr, 0, tm, a, sh); };
   const R* Mi0 = A.minv(0);
   // one sweep of level 0 after its row sums: f(node, X + om D^-1 (v - A X))
@@ -501,7 +565,7 @@ __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg,
       f(n, z);
     }
   };
-  R* at[CPFEM_MG_MAX_LEVELS];
+  R* at0;
   // ---- level 0, down
   {
     R *X = A.x(0), *T = A.t(0);
@@ -529,70 +593,16 @@ __device__ __noinline__ void mg_vcycle(const PointArgs& a, const cpfem_mg_t& mg,
       Res[3 * n0 + d] = (mg.free_dof != nullptr && mg.free_dof[3 * n0 + d] == 0) ? R(0) : rv;
     }
     barrier();
-    at[0] = X;
+    at0 = X;
   }
-  // ---- levels 1 .. lb-1, down
-  for (int l = 1; l < lb; ++l) {
-    const R* V = A.values(l);
-    const R* Mi = A.minv(l);
-    R *X = A.x(l), *T = A.t(l);
-    mgq_restrict(mg, l - 1, (const R*)A.r(l - 1), A.b(l), tq, sq, q);
-    mgq_first_sweep<TRANS>(mg, Mi, l, X, (const R*)A.b(l), tq, sq, q);
-    const int nsw = (l == L - 1) ? mg.coarse_sweeps : mg.pre_sweeps;
-    for (int k = 1; k < nsw; ++k) {
-      barrier();
-      mgq_apply<TRANS>(mg, V, Mi, l, (const R*)X, T, (const R*)A.b(l), false, tq, sq, q);
-      R* tmp = X; X = T; T = tmp;
-    }
-    at[l] = X;
-    if (l == L - 1) break;
-    barrier();
-    mgq_apply<TRANS>(mg, V, Mi, l, (const R*)X, A.r(l), (const R*)A.b(l), true, tq, sq, q);
-    barrier();
-  }
-  // ---- levels lb .. L-1: the dense operator.  Every block restricts the whole right-hand side
-  // (a few KB of residual, L1's work) rather than wait for its parts; a warp per row.
-  if (lb < L) {
-    R* b = reinterpret_cast<R*>(sh.part);
-    static_assert(sizeof(sh.part) >= sizeof(double) * 3 * kMgDenseNodes, "the dense right-hand side fits");
-    mgq_restrict(mg, lb - 1, (const R*)A.r(lb - 1), b, threadIdx.x >> 2, threads >> 2, q);
-    __syncthreads();
-    const int N = 3 * (int)mg.sell[lb].num_nodes;
-    const R* K = mg_dense<R>(mg);
-    R* X = A.x(lb);
-    const int r1 = (int)((int64_t)N * (rank + 1) / tm.nb);
-    for (int row = (int)((int64_t)N * rank / tm.nb) + wid; row < r1; row += warps) {
-      R acc = R(0);
-#pragma unroll 4
-      for (int c = lane; c < N; c += 32)
-        acc = mad(TRANS ? __ldg(&K[(size_t)c * N + row]) : __ldg(&K[(size_t)row * N + c]), b[c], acc);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) X[row] = acc;
-    }
-    at[lb] = X;
-  }
-  // ---- levels below the coarsest, up
-  for (int l = (lb < L ? lb : L - 1) - 1; l >= 1; --l) {
-    const R* V = A.values(l);
-    const R* Mi = A.minv(l);
-    R* X = at[l];
-    R* T = (X == A.x(l)) ? A.t(l) : A.x(l);
-    barrier();
-    if (q == 0) mg_prolong(mg, l, X, (const R*)at[l + 1], tq, sq, mg.sell[l].num_nodes);
-    for (int k = 0; k < mg.post_sweeps; ++k) {
-      barrier();
-      mgq_apply<TRANS>(mg, V, Mi, l, (const R*)X, T, (const R*)A.b(l), false, tq, sq, q);
-      R* tmp = X; X = T; T = tmp;
-    }
-    at[l] = X;
-  }
+  static_assert(sizeof(sh.part) >= sizeof(double) * 3 * kMgDenseNodes, "the dense right-hand side fits");
+  const R* X1 = mg_coarse_levels<TRANS, R>(mg, A, sh.lb, tq, sq, q, rank, tm.nb, reinterpret_cast<R*>(sh.part), barrier);
   // ---- level 0, up
   {
-    R* X = at[0];
+    R* X = at0;
     R* T = (X == A.x(0)) ? A.t(0) : A.x(0);
     barrier();
-    mg_prolong(mg, 0, X, (const R*)at[1], n0 + threadIdx.x, threads, n0 + nn);
+    mg_prolong(mg, 0, X, X1, n0 + threadIdx.x, threads, n0 + nn);
     auto finish = [&](int n, const R* z) {
 #pragma unroll
       for (int i = 0; i < 3; ++i) {

@@ -3,6 +3,7 @@
 // GB300): every mesh of the drop-in drivers and the RVEs of a batch.  Plans and launches.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 
 #include "krylov_team.cuh"
 
@@ -47,21 +48,35 @@ static int point_lanes(int64_t nodes, int blocks) {
 }
 
 // The rest of a plan, the lanes given: rows staged in shared memory where they fit (16 warps), else
-// read from L2 (24 warps, more loads in flight; what shared memory is left is L1's).  A transposed product that does so gathers its blocks from the neighbours' rows; past
-// 512 nodes a block the streaming kernel's four blocks per SM hide that better (48^3 cells, 774
-// nodes a block: 202 us per iteration here, 182 there; 40^3, 453 nodes: 115 and 129).
-static void point_fit(int64_t nodes, int blocks, int precond, bool transpose, bool teams, PointPlan* plan) {
+// read from L2 (24 warps, more loads in flight; what shared memory is left is L1's).
+//
+// Past some number of nodes a block the streaming kernel takes systems whose rows are not staged,
+// where it is the faster one.  A transposed product gathers its blocks from the neighbours' rows: a
+// block's range here is far from theirs, while the streaming kernel's blocks walk the mesh together
+// and find them in L2.  us per iteration, here and there, nodes a block in brackets:
+//   Jacobi transposed             40^3 cells (453) 115, 129     48^3 (774) 202, 182
+//   FP64 V-cycle transposed       36^3 (333) 465, 504           40^3 631, 561
+//   FP32 V-cycle transposed       44^3 (600) 529, 578           48^3 667, 661     52^3 (979) 990, 741
+//   FP32 V-cycle                  44^3 441, 462                 48^3 558, 539     52^3 652, 598
+//   FP64 V-cycle                  44^3 551, 633                 52^3 781, 911
+// so the last stays here as long as its vectors fit.
+static int64_t point_most(int precond, bool single, bool transpose) {
+  if (precond == 3) return single ? 700 : transpose ? 400 : INT64_MAX;
+  return transpose ? 512 : INT64_MAX;
+}
+
+static void point_fit(int64_t nodes, int blocks, int precond, bool single, bool transpose, bool teams, PointPlan* plan) {
   const int64_t npw = 32 / plan->lanes;
   const int64_t share = (ceil_div(ceil_div(nodes, npw), blocks) + (teams ? 1 : 0)) * npw;
   const size_t most = (size_t)kPtSmemBytes, vec = point_smem(share, precond, plan->lanes, false),
                all = point_smem(share, precond, plan->lanes, true);
   const bool staged = all <= most;
-  plan->ok = vec <= most && !(precond != 3 && transpose && !staged && share > 512);
+  plan->ok = vec <= most && (staged || share <= point_most(precond, single, transpose));
   plan->threads = precond == 3 ? kMgThreads : staged ? 512 : kPtMaxThreads;
   plan->smem_bytes = (int)std::max<size_t>(16, staged ? all : plan->ok ? vec : 0);
 }
 
-int point_plan(int64_t n, int precond, bool transpose, int grid_blocks, PointPlan* plan) {
+int point_plan(int64_t n, int precond, bool single, bool transpose, int grid_blocks, PointPlan* plan) {
   int sms = 0;
   const int rc = point_max_blocks(&sms);
   if (rc != CPFEM_OK) return rc;
@@ -71,13 +86,13 @@ int point_plan(int64_t n, int precond, bool transpose, int grid_blocks, PointPla
   plan->blocks = (int)blocks;
   plan->lanes = point_lanes(n, (int)blocks);
   if (precond == 3) plan->lanes = std::min(plan->lanes, 4);   // the V-cycle's kernels
-  point_fit(n, (int)blocks, precond, transpose, false, plan);
+  point_fit(n, (int)blocks, precond, single, transpose, false, plan);
   if (precond == 3 && plan->smem_bytes < (int)point_smem(ceil_div(n, blocks), precond, 1, true)) {
     // rows that stream: a unit of three rows per warp, as few lanes per node as keep most of
     // the eight warps at work
     plan->lanes = 1;
     while (plan->lanes < 4 && ceil_div(ceil_div(n, 32 / plan->lanes), blocks) < 6) plan->lanes *= 2;
-    point_fit(n, (int)blocks, precond, transpose, false, plan);
+    point_fit(n, (int)blocks, precond, single, transpose, false, plan);
   }
   return CPFEM_OK;
 }
@@ -85,7 +100,7 @@ int point_plan(int64_t n, int precond, bool transpose, int grid_blocks, PointPla
 int point_plan_teams(int64_t max_nodes_per_block, int precond, int blocks, PointPlan* plan) {
   plan->blocks = blocks;
   plan->lanes = point_lanes(max_nodes_per_block, 1);
-  point_fit(max_nodes_per_block, 1, precond, false, true, plan);
+  point_fit(max_nodes_per_block, 1, precond, false, false, true, plan);
   return CPFEM_OK;
 }
 

@@ -39,8 +39,6 @@ struct PointArgs {
   int true_res;                 // also form ||b - A x||^2 of the returned x
   double tol, atol;
   int smem_bytes;               // dynamic shared memory of a block
-  double* vectors[8];           // multigrid: the Krylov vectors (3 * num_nodes each) where they do not
-                                // fit in shared memory, else null
   int polls;                    // of a wait, at most
 };
 
@@ -54,16 +52,16 @@ struct PointPlan {
   int smem_bytes;
 };
 
-// Plan of one system of n nodes (grid_blocks > 0: that many blocks, at most one per SM).
-int point_plan(int64_t n, int precond, bool transpose, int grid_blocks, PointPlan* plan);
+// Plan of one system of n nodes (grid_blocks > 0: that many blocks, at most one per SM; single: the
+// V-cycle of precond 3 is FP32).
+int point_plan(int64_t n, int precond, bool single, bool transpose, int grid_blocks, PointPlan* plan);
 // Plan of teams whose largest share is max_nodes_per_block nodes.
 int point_plan_teams(int64_t max_nodes_per_block, int precond, int blocks, PointPlan* plan);
 // Blocks of a launch that can be resident together (one per SM).
 int point_max_blocks(int* blocks);
 int point_launch(const PointPlan& plan, bool transpose, PointArgs args, cudaStream_t s);
 
-// The V-cycle-preconditioned solve (krylov_mg.cu): a plan that is not ok streams its vectors
-// (args.vectors).
+// The V-cycle-preconditioned solve (krylov_mg.cu).
 int mg_launch(const PointPlan& plan, bool transpose, PointArgs args, const cpfem_mg_t& hierarchy, cudaStream_t s);
 int mg_check(const cpfem_mg_t* mg, const cpfem_sell_t* sell);
 

@@ -381,16 +381,6 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
   double* r = reinterpret_cast<double*>(pt_smem);
   double *rhat = r + nd, *p = rhat + nd, *q = p + nd, *t = q + nd, *xs = t + nd, *ph = xs + nd, *sh_ = ph + nd;
   double* minv = sh_ + nd;
-  bool resident = true;
-  if constexpr (kMg) {
-    // vectors too long for shared memory stay in the workspace
-    resident = a.vectors[0] == nullptr;
-    if (!resident) {
-      double** const vs[8] = {&r, &rhat, &p, &q, &t, &xs, &ph, &sh_};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) *vs[i] = a.vectors[i] + 3 * B.n0;
-    }
-  }
   if (threadIdx.x == 0) {
     sh.bad = 0;
     sh.steps = 0;
@@ -402,7 +392,7 @@ __global__ void __launch_bounds__(std::is_void<MR>::value ? kPtMaxThreads : kMgT
     atomicMax(&sh.steps, (a.L.group_width[(B.n0 + k) >> 5] + QL - 1) / QL);
   __syncthreads();
   B.steps = sh.steps;
-  const size_t vec_bytes = resident ? sizeof(double) * (8 * (size_t)nd + (size_t)mw * nn) : 0;
+  const size_t vec_bytes = sizeof(double) * (8 * (size_t)nd + (size_t)mw * nn);
   const size_t items = (size_t)B.units * B.steps * 32;
   B.staged = vec_bytes + items * (9 * sizeof(double) + sizeof(int)) <= (size_t)a.smem_bytes;
   B.mat = reinterpret_cast<double*>(pt_smem + vec_bytes);

@@ -35,7 +35,8 @@ def _lost(prob, A, b, x0, precond, mg, grid_blocks, deferred=False):
 # the shared-memory kernel over all SMs, and on seven blocks; the streaming kernel (12^3 nodes' vectors
 # do not fit one block's shared memory); both V-cycles
 @pytest.mark.parametrize("precond,mg,grid_blocks", [
-    (1, {}, 0), (2, {}, 7), (1, {}, 1), (3, {"precision": "fp64"}, 0), (3, {"precision": "fp32"}, 0)])
+    (1, {}, 0), (2, {}, 7), (1, {}, 1), (3, {"precision": "fp64"}, 0), (3, {"precision": "fp32"}, 0),
+    (3, {"precision": "fp64"}, 1), (3, {"precision": "fp32"}, 1)])
 def test_lost_block_ends_the_solve(pkg, gpu, precond, mg, grid_blocks):
     problem_mod, solver_mod = gpu
     prob, A, b, x0 = _system(pkg, problem_mod, solver_mod, (12, 12, 12))
