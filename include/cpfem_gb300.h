@@ -289,8 +289,10 @@ int cpfem_elem_assemble_ex(int32_t num_cells, const int32_t* cells, const double
 
 /* The assembly of cpfem_elem_assemble_ex over the whole mesh, gathered by node in one launch:
  * node n's cells are node_cells[node_ptr[n] .. node_ptr[n+1]), entries 8*cell + local node.
- * Values and residual are accumulated into, each by one thread in the order of the list, so
- * the result is bitwise reproducible.  Nodes of no cell are left as they are. */
+ * Values and residual are accumulated into without atomics: a value by one thread in the order of
+ * the list, a residual component in a fixed tree over its cells and points (another one without
+ * values on meshes above 20,000 nodes), so the result is bitwise reproducible.  Nodes of no cell
+ * are left as they are. */
 int cpfem_node_assemble(int32_t num_cells, int32_t num_nodes, const int32_t* node_ptr,
                         const int32_t* node_cells, const double* shape_grads,
                         const cpfem_sell_t* sell, const uint8_t* elem_pos,

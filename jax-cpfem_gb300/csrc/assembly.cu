@@ -521,6 +521,54 @@ k_node_assemble(int32_t num_nodes, const int32_t* __restrict__ node_ptr, const i
   }
 }
 
+// The residual alone on a large mesh: eight threads a node, one per GP, all three components, two
+// chains over the node's cells and a fixed tree over the points.  Bound by the FP64 pipe: 576 FMA a
+// node in 21 warp instructions, where k_node_assemble<false>'s 64 partial sums a component make
+// them 28.  On a small mesh that one's shorter chains are faster.  us a pass, that kernel and this
+// one: 20^3 cells 21, 25; 24^3 (15,625 nodes) 30, 32; 28^3 (24,389) 44, 34; 32^3 62, 49; 64^3 439,
+// 313 (345 by colours of cells).
+constexpr int kResThreads = 128;
+constexpr int32_t kResNodes = 20000;     // meshes above this use it
+
+__global__ void __launch_bounds__(kResThreads) k_node_residual(int32_t num_nodes, const int32_t* __restrict__ node_ptr,
+                                                               const int32_t* __restrict__ node_cells, int64_t G,
+                                                               const double* __restrict__ sg, const double* __restrict__ Pw,
+                                                               double* __restrict__ res) {
+  const int64_t na = (int64_t)blockIdx.x * (kResThreads / 8) + (threadIdx.x >> 3);
+  const int q = threadIdx.x & 7;
+  int n0 = 0, n1 = 0;
+  if (na < num_nodes) {
+    n0 = node_ptr[na];
+    n1 = node_ptr[na + 1];
+  }
+  double e[3] = {0.0, 0.0, 0.0}, o[3] = {0.0, 0.0, 0.0};     // the even and the odd cells of the list
+  auto cell = [&](int n, double* r) {
+    const int entry = __ldg(&node_cells[n]);                 // 8 cell + local node
+    const int64_t gp = (int64_t)(entry & ~7) + q;
+    const double* g = sg + gp * 24 + 3 * (entry & 7);
+    const double g0 = __ldg(&g[0]), g1 = __ldg(&g[1]), g2 = __ldg(&g[2]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      r[i] = fma(__ldg(&Pw[(3 * i) * G + gp]), g0,
+                 fma(__ldg(&Pw[(3 * i + 1) * G + gp]), g1, fma(__ldg(&Pw[(3 * i + 2) * G + gp]), g2, r[i])));
+  };
+  int n = n0;
+#pragma unroll 2
+  for (; n + 1 < n1; n += 2) {
+    cell(n, e);
+    cell(n + 1, o);
+  }
+  if (n < n1) cell(n, e);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    e[i] += o[i];
+#pragma unroll
+    for (int d = 4; d > 0; d >>= 1) e[i] += __shfl_xor_sync(0xFFFFFFFFu, e[i], d);
+  }
+  if (q < 3 && na < num_nodes) res[3 * na + q] += q == 0 ? e[0] : (q == 1 ? e[1] : e[2]);
+}
+
 // Row elimination for a list of unique Dirichlet dofs.
 __global__ void k_dirichlet(int32_t nbc, const int32_t* __restrict__ dofs, const double* __restrict__ bvals,
                             const double* __restrict__ u, double* __restrict__ res, const cpfem_sell_t L,
@@ -733,6 +781,12 @@ int cpfem_node_assemble(int32_t num_cells, int32_t num_nodes, const int32_t* nod
   };
   const size_t sm32 = sizeof(NodeShared<float>) * kBlockNodes, sm64 = sizeof(NodeShared<double>) * kBlockNodes;
   const double* t64 = static_cast<const double*>(tangent_w);
+  if (values == nullptr && residual != nullptr && num_nodes > kResNodes) {
+    k_node_residual<<<(unsigned)ceil_div(num_nodes, kResThreads / 8), kResThreads, 0, s>>>(num_nodes, node_ptr, node_cells, G,
+                                                                                         shape_grads, pk1_w, residual);
+    CPFEM_CUDA_TRY(cudaGetLastError());
+    return CPFEM_OK;
+  }
   if (values == nullptr) return run(k_node_assemble<false, double, double>, (const double*)nullptr, 0);
   if (k_precision == 0) return run(k_node_assemble<true, double, double>, t64, sm64);
   if (k_precision == 1) return run(k_node_assemble<true, float, double>, t64, sm32);
