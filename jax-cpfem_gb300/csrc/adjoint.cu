@@ -6,11 +6,15 @@
 
 namespace cpfem {
 
-constexpr int kVjpK = 4;   // tangent directions per dual sweep
-constexpr int kVjpThreads = 64;
+// Tangent directions per dual sweep: the six of s, and the nine of F, are whole sweeps of three.  The
+// FP64 pipe bounds the kernel (64 cycles per warp instruction, some 8,000 a sweep).  ms for the two
+// passes of two steps, 8,000 points, 12 systems: 5.8 (four directions: 6.4; the kernel before, slip
+// systems unrolled, sweeps of four seeded through an index array: 6.0); 4,096 points of 24: 13.3
+// (13.6; 17.7).
+constexpr int kVjpK = 3;
 
 template <int NS>
-__global__ void __launch_bounds__(kVjpThreads) k_gp_vjp(const __grid_constant__ MatDev m, const cpfem_vjp_args_t a) {
+__global__ void __launch_bounds__(64) k_gp_vjp(const __grid_constant__ MatDev m, const cpfem_vjp_args_t a) {
   const int64_t gp = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t G = a.num_gp;
   if (gp >= G) return;
@@ -40,7 +44,7 @@ __global__ void __launch_bounds__(kVjpThreads) k_gp_vjp(const __grid_constant__ 
 #pragma unroll
       for (int J = 0; J < 3; ++J) F[3 * i + J] = fma(a.u[3 * nb + i], sg[3 * b + J], F[3 * i + J]);
   }
-  double Fpi[9], R[9], th[5], g[NS];
+  double Fpi[9], R[9], th[5];
 #pragma unroll
   for (int k = 0; k < 9; ++k) Fpi[k] = a.fpi[k * G + gp];
 #pragma unroll
@@ -53,43 +57,36 @@ __global__ void __launch_bounds__(kVjpThreads) k_gp_vjp(const __grid_constant__ 
     cc.C12 = a.elastic_table[3 * pi + 1];
     cc.C44 = a.elastic_table[3 * pi + 2];
   }
-#pragma unroll
-  for (int s = 0; s < NS; ++s) {
-    g[s] = a.g[s * G + gp];
-    GpSlab<NS, kVjpThreads>::ig(s) = 1.0 / g[s];
-  }
+  auto g = [&](int s) { return a.g[s * G + gp]; };
   // recompute the converged local state from the checkpoint (u, Fp^-1, g and, if kept,
   // the converged S as the local Newton's start)
-  double A[9], AR[9], Ct[9];
-  mm3(F, Fpi, A);
-  mm3(A, R, AR);
-  mm3_at(AR, AR, Ct);
   const double cdt = m.ao * a.dt;
-  GPSolve st;
-  double s0[6];
-  if (a.s_start != nullptr)
+  double s[6], rn;
+  {
+    double A[9], AR[9], Ct[9];
+    mm3(F, Fpi, A);
+    mm3(A, R, AR);
+    mm3_at(AR, AR, Ct);
+    const bool warm = a.s_start != nullptr;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) s0[k] = a.s_start[k * G + gp];
-  cp_local_newton<NS, kVjpThreads>(m, cc, Ct, cdt, 1.0 / th[3], st, a.s_start != nullptr ? s0 : nullptr);
+    for (int k = 0; k < 6; ++k) s[k] = warm ? a.s_start[k * G + gp] : 0.0;
+    rn = cp_root<NS>(m, cc, Ct, cdt, 1.0 / th[3], g, warm, s);
+  }
   // output cotangents
-  constexpr int NY = YOut<NS>::kN;
-  double ybar[NY];
+  YBar ybar;
 #pragma unroll
-  for (int o = 0; o < NY; ++o) ybar[o] = 0.0;
+  for (int c = 0; c < 9; ++c) {
+    ybar.P[c] = ybar.sig[c] = 0.0;
+    ybar.Fp[c] = (a.fpi_bar != nullptr) ? a.fpi_bar[c * G + gp] : 0.0;
+  }
   if (a.cell_sig_bar != nullptr) {
     double wsum = 0.0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) wsum += a.jxw[e * 8 + q];
     const double wq = a.jxw[gp] / wsum;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) ybar[YOut<NS>::kSig + c] = a.cell_sig_bar[e * 9 + c] * wq;
+    for (int c = 0; c < 9; ++c) ybar.sig[c] = a.cell_sig_bar[e * 9 + c] * wq;
   }
-  if (a.fpi_bar != nullptr)
-#pragma unroll
-    for (int c = 0; c < 9; ++c) ybar[YOut<NS>::kFp + c] = a.fpi_bar[c * G + gp];
-  if (a.g_bar != nullptr)
-#pragma unroll
-    for (int s = 0; s < NS; ++s) ybar[YOut<NS>::kG + s] = a.g_bar[s * G + gp];
   if (a.mode == 2 && a.mu != nullptr) {
     // P cotangent of the equilibrium term: -JxW * grad(mu)
     const double w = a.jxw[gp];
@@ -99,44 +96,24 @@ __global__ void __launch_bounds__(kVjpThreads) k_gp_vjp(const __grid_constant__ 
 #pragma unroll
       for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int J = 0; J < 3; ++J)
-          ybar[YOut<NS>::kP + 3 * i + J] = fma(-w * a.mu[3 * nb + i], sg[3 * b + J], ybar[YOut<NS>::kP + 3 * i + J]);
+        for (int J = 0; J < 3; ++J) ybar.P[3 * i + J] = fma(-w * a.mu[3 * nb + i], sg[3 * b + J], ybar.P[3 * i + J]);
     }
   }
-  constexpr int NX = XIn<NS>::kN;
-  double xbar[NX];
-  int dirs[NX];
-  int ndir = 0;
-  if (a.mode == 1) {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) dirs[ndir++] = XIn<NS>::kF + k;
-  } else {
-    for (int k = XIn<NS>::kFp; k < NX; ++k) dirs[ndir++] = k;
-  }
-  const bool ok = cp_vjp<NS, kVjpK>(m, cc, cdt, st.s, F, Fpi, g, R, th, ybar, dirs, ndir, xbar);
+  auto gbar = [&](int s) { return (a.g_bar != nullptr) ? a.g_bar[s * G + gp] : 0.0; };
+  // the cotangent of input idx goes to its place, where the caller wants it
+  using X = XIn<NS>;
+  auto out = [&](int idx, double v) {
+    double* p = idx < X::kFp ? a.f_bar : idx < X::kG ? a.fpi_bar_old : idx < X::kTh ? a.g_bar_old : idx < X::kW ? a.theta_bar : a.rot_bar;
+    const int at = idx - (idx < X::kFp ? X::kF : idx < X::kG ? X::kFp : idx < X::kTh ? X::kG : idx < X::kW ? X::kTh : X::kW);
+    if (p != nullptr) p[at * G + gp] = v;
+  };
+  const bool ok = cp_vjp<NS, kVjpK>(m, cc, cdt, s, F, Fpi, R, th, g, ybar, gbar, a.mode == 1 ? X::kF : X::kFp,
+                                    a.mode == 1 ? X::kFp : X::kN, out);
   if (a.status != nullptr) {
     int bits = 0;
-    if (!(st.rn <= m.local_tol)) bits |= CPFEM_GP_MAXITER;
-    if (!ok || !isfinite(st.rn)) bits |= CPFEM_GP_NONFINITE;
+    if (!(rn <= m.local_tol)) bits |= CPFEM_GP_MAXITER;
+    if (!ok || !isfinite(rn)) bits |= CPFEM_GP_NONFINITE;
     if (bits) atomicOr(a.status, bits);
-  }
-  if (a.mode == 1) {
-    if (a.f_bar != nullptr)
-#pragma unroll
-      for (int k = 0; k < 9; ++k) a.f_bar[k * G + gp] = xbar[XIn<NS>::kF + k];
-  } else {
-    if (a.fpi_bar_old != nullptr)
-#pragma unroll
-      for (int k = 0; k < 9; ++k) a.fpi_bar_old[k * G + gp] = xbar[XIn<NS>::kFp + k];
-    if (a.g_bar_old != nullptr)
-#pragma unroll
-      for (int s = 0; s < NS; ++s) a.g_bar_old[s * G + gp] = xbar[XIn<NS>::kG + s];
-    if (a.theta_bar != nullptr)
-#pragma unroll
-      for (int k = 0; k < 5; ++k) a.theta_bar[k * G + gp] = xbar[XIn<NS>::kTh + k];
-    if (a.rot_bar != nullptr)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) a.rot_bar[k * G + gp] = xbar[XIn<NS>::kW + k];
   }
 }
 
@@ -157,22 +134,23 @@ extern "C" int cpfem_gp_vjp(const cpfem_material_t* mat, const cpfem_vjp_args_t*
                     a.param_table, "input pointer is null");
   CPFEM_REQUIRE(md.qmode == 0 || md.num_slip % 3 == 0, "qmode 1 needs num_slip % 3 == 0");
   CPFEM_REQUIRE(a.num_nodes > 0 && a.num_rot > 0 && a.num_param > 0, "table sizes must be given");
-  const unsigned blocks = (unsigned)ceil_div(a.num_gp, kVjpThreads);
+  const int threads = 64;
+  const unsigned blocks = (unsigned)ceil_div(a.num_gp, threads);
   cudaStream_t s = (cudaStream_t)stream;
   const void* fn = (md.num_slip == 12) ? (const void*)k_gp_vjp<12> : (const void*)k_gp_vjp<24>;
   // the dual-number sweeps need a large per-thread stack: make sure the limit covers it
   cudaFuncAttributes attr;
   CPFEM_CUDA_TRY(cudaFuncGetAttributes(&attr, fn));
+  // (the builds with another frame faulted, gp_adjoint.cuh)
+  CPFEM_REQUIRE(attr.localSizeBytes % 32 == 0, "the backward kernel was built with a stack frame that is no multiple of 32");
   size_t limit = 0;
   CPFEM_CUDA_TRY(cudaDeviceGetLimit(&limit, cudaLimitStackSize));
   const size_t need = attr.localSizeBytes + 1024;
   if (limit < need) CPFEM_CUDA_TRY(cudaDeviceSetLimit(cudaLimitStackSize, need));
-  const size_t smem = md.num_slip == 12 ? GpSlab<12, kVjpThreads>::kBytes : GpSlab<24, kVjpThreads>::kBytes;
-  CPFEM_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (md.num_slip == 12)
-    k_gp_vjp<12><<<blocks, kVjpThreads, smem, s>>>(md, a);
+    k_gp_vjp<12><<<blocks, threads, 0, s>>>(md, a);
   else
-    k_gp_vjp<24><<<blocks, kVjpThreads, smem, s>>>(md, a);
+    k_gp_vjp<24><<<blocks, threads, 0, s>>>(md, a);
   CPFEM_CUDA_TRY(cudaGetLastError());
   return CPFEM_OK;
 }
