@@ -457,13 +457,14 @@ typedef struct {
 
 typedef struct {
   int32_t precond;        /* 0 none, 1 Jacobi (the reference), 2 3x3 block-Jacobi, 3 multigrid */
-  int32_t transpose;      /* solve A^T x = b (precond 0..2) */
+  int32_t transpose;      /* solve A^T x = b */
   int32_t maxiter;
   int32_t max_restarts;
   double tol, atol;
   const cpfem_mg_t* mg;   /* precond 3: a hierarchy set up for this matrix */
-  int32_t grid_blocks;    /* blocks of the persistent launch; 0: one per 256 nodes, at most the
-                             co-resident limit (larger requests are clamped to it) */
+  int32_t grid_blocks;    /* blocks of the persistent launch, at most what can be resident
+                             together (larger requests are clamped); 0: by size, one per SM
+                             where the vectors fit its shared memory */
   int32_t flags;          /* bit 0: also form ||b - A x||^2 of the returned x in the same launch
                              (cpfem_bicgstab_last_stats_ex), for the caller's true-residual check;
                              bit 1: deferred report -- the call queues the copy of the launch's

@@ -2,8 +2,9 @@
 
 The multigrid-preconditioned BiCGSTAB has settings whose best values depend on the mesh
 size, the material state and the GPU: the number of levels, the smoothing sweeps and
-damping, and the grid size of the persistent launch (more blocks hide latency in the
-SpMVs, fewer make each grid barrier cheaper).  ``tune_linear_solver`` times complete
+damping, whether the small coarse levels become a dense operator (``local_nodes``, 256 at
+most), and the blocks of the persistent launch (0: one per SM; fewer make each grid barrier
+cheaper).  ``tune_linear_solver`` times complete
 solves of a real Newton system (CUDA events on the solve's stream, after one untimed
 solve per configuration) with a coordinate search over those settings, and returns the
 fastest configuration that converged.  Every candidate solves the same system to the
@@ -28,8 +29,8 @@ SEARCH = (("precision", ("fp64", "fp32")),
           ("post_sweeps", (0, 1, 2)),
           ("coarse_sweeps", (4, 8, 12)),
           ("max_levels", (3, 4, 5)),
-          ("local_nodes", (256, 1024)),
-          ("grid_blocks", (0, 76, 104, 152, 304)))
+          ("local_nodes", (256, 1)),
+          ("grid_blocks", (0, 76, 104)))
 
 
 def _time_solve(problem, A, b, x0, cfg, reps, tol=1e-10):
