@@ -991,9 +991,9 @@ __global__ void __launch_bounds__(kPThreads, 4) k_bicgstab_ragged(
   }
 }
 
-// Teams of the shared-memory kernel, one per job: every job's share of the blocks by weight
-// (at least one block, at most one per kMinPointNodes nodes).  Not used (plan->ok = false)
-// where that leaves a job's vectors too large for its blocks, or with more than half as many
+// Teams of the shared-memory kernel, one per job: a block each, and then one after another to the
+// team with the most work per block (at most one per kMinPointNodes nodes).  Not used (plan->ok =
+// false) where that leaves a job's vectors too large for its blocks, or with more than half as many
 // jobs as SMs: then the FP64 pipe is busy anyway and the streaming kernel's four blocks per
 // SM hide more latency.
 constexpr int64_t kMinPointNodes = 16;
@@ -1006,18 +1006,25 @@ static int ragged_point_plan(const std::vector<RJob>& jobs, const std::vector<do
   if (rc != CPFEM_OK) return rc;
   const int nj = (int)jobs.size();
   if (2 * nj > sms) return CPFEM_OK;
-  double wsum = 0.0;
-  for (double v : wts) wsum += v;
+  auto nodes = [&](int j) { return jobs[(size_t)j].n1 - jobs[(size_t)j].n0; };
+  std::vector<int64_t> k((size_t)nj, 1);
+  for (int left = sms - nj; left > 0; --left) {
+    int best = -1;
+    for (int j = 0; j < nj; ++j)
+      if (k[(size_t)j] < ceil_div(nodes(j), kMinPointNodes) &&
+          (best < 0 || wts[(size_t)j] / (double)k[(size_t)j] > wts[(size_t)best] / (double)k[(size_t)best]))
+        best = j;
+    if (best < 0) break;
+    k[(size_t)best] += 1;
+  }
   int next = 0;
   int64_t share = 0;
   for (int j = 0; j < nj; ++j) {
-    const int64_t n = jobs[(size_t)j].n1 - jobs[(size_t)j].n0;
-    int64_t k = 1 + (int64_t)std::floor((double)(sms - nj) * wts[(size_t)j] / wsum);
-    k = std::min<int64_t>(k, std::max<int64_t>(1, ceil_div(n, kMinPointNodes)));
-    teams->push_back(PointTeam{next, (int)k, j, 0, jobs[(size_t)j].n0, jobs[(size_t)j].n1});
-    for (int64_t c = 0; c < k; ++c) team_of_block->push_back(j);
-    next += (int)k;
-    share = std::max(share, ceil_div(n, k));
+    const int nb = (int)k[(size_t)j];
+    teams->push_back(PointTeam{next, nb, j, 0, jobs[(size_t)j].n0, jobs[(size_t)j].n1});
+    team_of_block->insert(team_of_block->end(), (size_t)nb, j);
+    next += nb;
+    share = std::max(share, ceil_div(nodes(j), (int64_t)nb));
   }
   const int prc = point_plan_teams(share, precond, next, plan);
   if (prc != CPFEM_OK || !plan->ok) {
