@@ -41,18 +41,10 @@ __device__ __forceinline__ void mg_apply_minv(const R* __restrict__ minv, int64_
   }
 }
 
-// A value of a level operator: read-only for the whole launch, so through the read-only
-// cache from global memory, or a plain load from shared memory (SH).
-template <bool SH, typename R>
-__device__ __forceinline__ R ldc(const R* p) {
-  if constexpr (SH) return *p;
-  else return __ldg(p);
-}
-
 // Rows of node a of A x (A^T x when TRANS) restricted to the slots j = q (mod 4) (one lane of
 // a quad).  x by plain loads: shared memory, or global memory whose writers the grid's last
 // barrier ordered (neighbours share values, which L1 then serves).
-template <bool TRANS, typename R, bool SHV = false>
+template <bool TRANS, typename R>
 __device__ __forceinline__ void sell_rows_quad(const cpfem_sell_t& L, const R* __restrict__ vals, const R* x,
                                                int64_t a, int q, R* acc) {
   const int64_t g = a >> 5;
@@ -67,15 +59,15 @@ __device__ __forceinline__ void sell_rows_quad(const cpfem_sell_t& L, const R* _
     const R x0 = x[3 * b], x1 = x[3 * b + 1], x2 = x[3 * b + 2];
     if (!TRANS) {
       const R* vb = v0 + 288 * j;
-      a0 = mad(ldc<SHV>(&vb[0]), x0, mad(ldc<SHV>(&vb[32]), x1, mad(ldc<SHV>(&vb[64]), x2, a0)));
-      a1 = mad(ldc<SHV>(&vb[96]), x0, mad(ldc<SHV>(&vb[128]), x1, mad(ldc<SHV>(&vb[160]), x2, a1)));
-      a2 = mad(ldc<SHV>(&vb[192]), x0, mad(ldc<SHV>(&vb[224]), x1, mad(ldc<SHV>(&vb[256]), x2, a2)));
+      a0 = mad(__ldg(&vb[0]), x0, mad(__ldg(&vb[32]), x1, mad(__ldg(&vb[64]), x2, a0)));
+      a1 = mad(__ldg(&vb[96]), x0, mad(__ldg(&vb[128]), x1, mad(__ldg(&vb[160]), x2, a1)));
+      a2 = mad(__ldg(&vb[192]), x0, mad(__ldg(&vb[224]), x1, mad(__ldg(&vb[256]), x2, a2)));
     } else {
       const int64_t tp = __ldg(&L.tpos[c0 + 32 * j]);
       const R* vb = vals + 9 * L.group_off[b >> 5] + (b & 31) + 288 * tp;
-      a0 = mad(ldc<SHV>(&vb[0]), x0, mad(ldc<SHV>(&vb[96]), x1, mad(ldc<SHV>(&vb[192]), x2, a0)));
-      a1 = mad(ldc<SHV>(&vb[32]), x0, mad(ldc<SHV>(&vb[128]), x1, mad(ldc<SHV>(&vb[224]), x2, a1)));
-      a2 = mad(ldc<SHV>(&vb[64]), x0, mad(ldc<SHV>(&vb[160]), x1, mad(ldc<SHV>(&vb[256]), x2, a2)));
+      a0 = mad(__ldg(&vb[0]), x0, mad(__ldg(&vb[96]), x1, mad(__ldg(&vb[192]), x2, a0)));
+      a1 = mad(__ldg(&vb[32]), x0, mad(__ldg(&vb[128]), x1, mad(__ldg(&vb[224]), x2, a1)));
+      a2 = mad(__ldg(&vb[64]), x0, mad(__ldg(&vb[160]), x1, mad(__ldg(&vb[256]), x2, a2)));
     }
   }
   acc[0] = a0;
@@ -95,16 +87,15 @@ __host__ __device__ constexpr int64_t st_idx_index(int64_t i) { return i + kStSk
 constexpr int64_t kStValRow = 288 + kStSkew, kStIdxRow = 32 + kStSkew;
 
 // sell_rows_quad on a level staged in shared memory: values, x and the index tables
-// (group offsets, widths, columns, transposed slots as int32, mg_stage) all there, the
-// values and the column / transposed-slot tables in the skewed order above (group offsets
-// are multiples of 32 slots, so a group's rows start at a whole skewed row).
-template <bool TRANS, typename R>
+// (group offsets, widths and columns as int32, mg_stage) all there, the values and the columns in
+// the skewed order above (group offsets are multiples of 32 slots, so a group's rows start at a
+// whole skewed row).
+template <typename R>
 __device__ __forceinline__ void sell_rows_quad_st(const int* ix, int ng, const R* vals, const R* x, int64_t a,
                                                   int q, R* acc) {
   const int* goff = ix;
   const int* gw = ix + ng + 1;
   const int* cols = gw + ng;
-  const int* tpos = cols + kStIdxRow * kMgMaxWidth * ng;
   const int g = (int)(a >> 5);
   const int lane = (int)(a & 31);
   const int gs = goff[g];
@@ -116,19 +107,10 @@ __device__ __forceinline__ void sell_rows_quad_st(const int* ix, int ng, const R
   for (int j = q; j < w; j += 4) {
     const int b = cols[c0 + (int)kStIdxRow * j];
     const R x0 = x[3 * b], x1 = x[3 * b + 1], x2 = x[3 * b + 2];
-    if (!TRANS) {
-      const R* vb = v0 + kStValRow * j;
-      a0 = mad(vb[0], x0, mad(vb[32], x1, mad(vb[64], x2, a0)));
-      a1 = mad(vb[96], x0, mad(vb[128], x1, mad(vb[160], x2, a1)));
-      a2 = mad(vb[192], x0, mad(vb[224], x1, mad(vb[256], x2, a2)));
-    } else {
-      const int tp = tpos[c0 + (int)kStIdxRow * j];
-      const int gb = goff[b >> 5];
-      const R* vb = vals + 9 * gb + (int)kStSkew * (gb >> 5) + (b & 31) + kStValRow * tp;
-      a0 = mad(vb[0], x0, mad(vb[96], x1, mad(vb[192], x2, a0)));
-      a1 = mad(vb[32], x0, mad(vb[128], x1, mad(vb[224], x2, a1)));
-      a2 = mad(vb[64], x0, mad(vb[160], x1, mad(vb[256], x2, a2)));
-    }
+    const R* vb = v0 + kStValRow * j;
+    a0 = mad(vb[0], x0, mad(vb[32], x1, mad(vb[64], x2, a0)));
+    a1 = mad(vb[96], x0, mad(vb[128], x1, mad(vb[160], x2, a1)));
+    a2 = mad(vb[192], x0, mad(vb[224], x1, mad(vb[256], x2, a2)));
   }
   acc[0] = a0;
   acc[1] = a1;
@@ -200,7 +182,7 @@ __device__ __forceinline__ void mgq_apply(const cpfem_mg_t& mg, const R* V, cons
   for (int64_t a = tq; a < npad; a += sq) {
     R acc[3] = {R(0), R(0), R(0)};
     if (a < n) {
-      if constexpr (SHV) sell_rows_quad_st<TRANS>(sidx, S.num_groups, V, X, a, q, acc);
+      if constexpr (SHV) sell_rows_quad_st(sidx, S.num_groups, V, X, a, q, acc);
       else sell_rows_quad<TRANS, R>(S, V, X, a, q, acc);
     }
     quad_sum3(acc);
@@ -359,16 +341,15 @@ struct MgShared {
   size_t vec[CPFEM_MG_MAX_LEVELS];
   size_t val[CPFEM_MG_MAX_LEVELS];
   size_t minv[CPFEM_MG_MAX_LEVELS];
-  size_t idx[CPFEM_MG_MAX_LEVELS];   // int32: group offsets, group widths, columns, transposed slots
+  size_t idx[CPFEM_MG_MAX_LEVELS];   // int32: group offsets, group widths, columns
   size_t total;
   bool staged;
 };
 
-// int32 entries of a staged level's layout: ng+1 group offsets, ng widths, and the column
-// and transposed-slot tables of 32 * kMgMaxWidth slots per group (skewed: kStIdxRow words
-// per slot row)
+// int32 entries of a staged level's layout: ng+1 group offsets, ng widths, and the columns of
+// 32 * kMgMaxWidth slots per group (skewed: kStIdxRow words per slot row)
 __host__ __device__ inline size_t mg_idx_words(int32_t ng) {
-  return 2 * (size_t)ng + 1 + 2 * (size_t)kStIdxRow * (size_t)kMgMaxWidth * ng;
+  return 2 * (size_t)ng + 1 + (size_t)kStIdxRow * (size_t)kMgMaxWidth * ng;
 }
 
 __host__ __device__ inline MgShared mg_shared_layout(const cpfem_mg_t& mg, int lb, size_t real_bytes) {
@@ -414,13 +395,9 @@ __device__ bool mg_stage(const cpfem_mg_t& mg, int lb, const MgArrays<R>& A, con
     const int ng = S.num_groups;
     const int64_t ns = S.group_off[ng];
     int* cols = ix + 2 * ng + 1;
-    int* tpos = cols + kStIdxRow * kMgMaxWidth * ng;
     for (int64_t i = threadIdx.x; i <= ng; i += blockDim.x) ix[i] = (int)S.group_off[i];
     for (int64_t i = threadIdx.x; i < ng; i += blockDim.x) ix[ng + 1 + i] = S.group_width[i];
-    for (int64_t i = threadIdx.x; i < ns; i += blockDim.x) {
-      cols[st_idx_index(i)] = S.cols[i];
-      tpos[st_idx_index(i)] = (S.tpos != nullptr) ? S.tpos[i] : 0;
-    }
+    for (int64_t i = threadIdx.x; i < ns; i += blockDim.x) cols[st_idx_index(i)] = S.cols[i];
   }
   __syncthreads();
   return true;
