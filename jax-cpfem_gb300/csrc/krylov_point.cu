@@ -1,6 +1,7 @@
 // Persistent BiCGSTAB with the point preconditioners (none, 1/diag, inverted 3x3 diagonal
 // block) for systems whose Krylov vectors fit in shared memory (up to about 53^3 cells on one
-// GB300): every mesh of the drop-in drivers and the RVEs of a batch.  Plans and launches.
+// GB300): every mesh of the drop-in drivers and the RVEs of a batch.  Plans (the multigrid solve's
+// too) and launches.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>

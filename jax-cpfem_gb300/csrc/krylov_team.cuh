@@ -9,7 +9,7 @@
 //    takes one of the three rows of 32 / QL consecutive nodes, and QL lanes share a row's
 //    neighbour slots.  With one thread per node a 10^3 mesh ran on 6 SMs.
 //  * every vector but the two that neighbours gather lives in the block's shared memory, and
-//    so do, where they fit, the block's matrix rows and column indices (up to ~22^3 cells),
+//    so do, where they fit, the block's matrix rows and column indices (up to ~21^3 cells),
 //    copied once per solve.  A transposed solve copies the transposed rows, so its product
 //    reads shared memory in order like any other.
 //  * FP64 instructions are spent where there is data: one lane computes the scalars, one
