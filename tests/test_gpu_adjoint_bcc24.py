@@ -1,5 +1,6 @@
-"""The backward kernel for 24 slip systems: the gradient of a load history against complex-step
-derivatives of the oracle's, as for 12."""
+"""The backward kernel where its loops and branches differ: 24 slip systems, hardening without
+coplanar blocks, a non-integer hardening exponent -- the gradient of a load history against
+complex-step derivatives of the oracle's."""
 import importlib
 
 import numpy as np
@@ -8,12 +9,15 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,grains,steps", [(1, 1, 1), (2, 3, 2)])
-def test_adjoint_of_24_systems_matches_oracle_complex_step(pkg, gpu, n, grains, steps):
+@pytest.mark.parametrize("spec_name,changes,n,grains,steps", [
+    ("BENCH_TANTALUM", {}, 1, 1, 1), ("BENCH_TANTALUM", {}, 2, 3, 2), ("BENCH_TANTALUM", {"coplanar_q": False}, 2, 3, 2),
+    ("BENCH_STEEL", {"coplanar_q": False, "gss_a": 2.5}, 2, 3, 2)])
+def test_adjoint_matches_oracle_complex_step(pkg, gpu, spec_name, changes, n, grains, steps):
     from oracle import cpfem_oracle as O
     problem_mod, _ = gpu
     adjoint = importlib.import_module("jax-cpfem_gb300.adjoint")
-    spec = pkg.material.BENCH_TANTALUM.replace(local_tol=1e-10)
+    spec = getattr(pkg.material, spec_name).replace(local_tol=1e-10, **changes)
+    table = O.BCC24 if spec.num_slip == 24 else O.FCC12
     mesh = pkg.box_mesh(n, n, n)
     ori, rng = pkg.mesh.voronoi_grains(mesh, grains, 4)
     quat = pkg.material.random_quaternions(rng, grains)
@@ -33,7 +37,7 @@ def test_adjoint_of_24_systems_matches_oracle_complex_step(pkg, gpu, n, grains, 
 
     def f(theta, euler):
         bcs = lambda d: [(nodes, c, v) for nodes, c, v in zip(faces, (0, 1, 2, 2), (0.0, 0.0, 0.0, d))]
-        return O.history_stress(p, mesh.cells, O.BCC24, (spec.C11, spec.C12, spec.C44), quat, ori, theta, euler,
+        return O.history_stress(p, mesh.cells, table, (spec.C11, spec.C12, spec.C44), quat, ori, theta, euler,
                                 h.disps, h.ts, bcs, r=spec.r, coplanar=spec.coplanar_q, ao=spec.ao,
                                 local_tol=spec.local_tol, max_sub_step=spec.max_sub_step,
                                 solver_options={"tol": 1e-10, "rel_tol": 1e-13, "max_newton": 40})[:, 2, 2]
